@@ -36,3 +36,27 @@ def test_householder_panels_at_the_edges_of_their_layouts(ext, n, k):
     assert float((Q.T @ Q - eye).abs().max()) < bound
     R = torch.triu(ct.double().T[:k])
     assert float((Q[:, :k] @ R - Y.float().double()).norm() / Y.norm()) < bound
+
+
+# Blocks of four columns, an even number of them: the sizes around their edges, and repeated or zero eigenvalues.
+@pytest.mark.parametrize("n", [3, 4, 5, 8, 9, 12, 31, 33, 97, 124, 125, 127])
+@pytest.mark.parametrize("kind", ["full", "identity", "low_rank", "graded"])
+def test_jacobi_blocks_at_their_edges(ext, n, kind):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    B = torch.randn(n, 2 * n, device="cuda", generator=gen, dtype=torch.float64)
+    A = {
+        "full": B @ B.T / n,
+        "identity": 3.0 * torch.eye(n, device="cuda", dtype=torch.float64),
+        "low_rank": B[:, :2] @ B[:, :2].T + 1e-6 * torch.eye(n, device="cuda", dtype=torch.float64),
+        "graded": B @ B.T / n * torch.logspace(0, -3, n, device="cuda", dtype=torch.float64).outer(torch.logspace(0, -3, n, device="cuda", dtype=torch.float64)),
+    }[kind].float()
+    lams, qs, sweeps = ext.jacobi_eigh([A], 24, 2e-6)
+    assert int(sweeps[0]) <= 24
+    want = torch.linalg.eigvalsh(A.double())
+    scale = float(want.abs().max())
+    # a column takes part in n rotations a sweep, in about 15 sweeps, and c^2 + s^2 is off by up to 2^-24 each time
+    bound = (15 * n + 16) * 2.0**-24
+    assert float((lams[0].double() - want).abs().max()) < bound * scale
+    Q = qs[0].double()
+    assert float((Q.T @ Q - torch.eye(n, device="cuda", dtype=torch.float64)).abs().max()) < 5e-6
+    assert float(((Q * lams[0].double()) @ Q.T - A.double()).abs().max()) < bound * scale
