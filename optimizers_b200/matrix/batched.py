@@ -304,16 +304,19 @@ def eigdec_refresh_supported(cfg: Any) -> bool:
     )
 
 
-def batched_eigen_refresh(ext: Any, blocks: list[Any], bias_correction2: Tensor | float, split: bool, status: Tensor) -> None:
+def batched_eigen_refresh(
+    ext: Any, blocks: list[Any], bias_correction2: Tensor | float, split: bool, status: Tensor
+) -> list[tuple[Any, int]]:
     """Refresh ``inv_factor_matrices`` (state) and the ``inv_hi/inv_lo`` mirrors of ``blocks``.
     For eigendecomposed Shampoo (``factors.kind == "eigendecomposed"``) the state refreshed is the
-    pair (eigenvalues, eigenvectors) and the mirrors receive the reconstruction, split in place.
+    pair (eigenvalues, eigenvectors) and the mirrors receive the reconstruction, split in place where the
+    block has an ``inv_lo``.  Returns the ``(block, k)`` whose ``inv_hi`` was written.
 
     ``blocks`` are the native engine's block records (``.factors`` is the ``BlockFactors`` of the
     block, ``.inv_hi/.inv_lo`` the mirrors).  Raises ``PreconditionerValueError`` on non-finite
     factors or results and ``ValueError`` once a block exceeds its tolerated failures."""
     if not blocks:
-        return
+        return []
     device = blocks[0].inv_hi[0].device
     main = torch.cuda.current_stream(device)
 
@@ -514,7 +517,7 @@ def batched_eigen_refresh(ext: Any, blocks: list[Any], bias_correction2: Tensor 
             kf.factor_matrices_eigenvectors[it.k].copy_(it.Q)
             mirror = it.block.inv_hi[it.k][:, :d]
             checked.append(mirror)  # finite only if the eigenvalues it was built from are
-            if split:  # the reconstruction becomes the (hi, lo) operand pair in place
+            if split and it.block.inv_lo[it.k] is not None:  # the reconstruction becomes the (hi, lo) operand pair in place
                 ext.tf32_split(mirror, mirror, it.block.inv_lo[it.k][:, :d])
             continue
         state = kf.inv_factor_matrices[it.k]
@@ -549,6 +552,7 @@ def batched_eigen_refresh(ext: Any, blocks: list[Any], bias_correction2: Tensor 
             last_error.setdefault(id(it.block), None)
     for b in blocks:
         b.factors.note_refresh_outcome(last_error.get(id(b)))
+    return [(it.block, it.k) for it in good]
 
 
 # ----------------------------------------------------------------------------------------------

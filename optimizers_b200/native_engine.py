@@ -76,6 +76,12 @@ def _pad4(n: int) -> int:
     return (n + 3) // 4 * 4
 
 
+# Step scratch of one block: two norms, then the (bound, squared row norm) meta data of its half-pair operands.
+# The first three slots are read by the kernels under these offsets (block_kernels.cuh, kMeta*).
+_META_GRAD, _META_FILTERED, _META_SCALED, _META_T, _META_T2, _META_U, _META_U2 = range(0, 14, 2)
+_META_SIZE = 14
+
+
 # Configurations whose 2-D blocks may carry a factor on one dim only (the other switched off by an
 # exponent of 0): one-sided products.  Under KL-Shampoo such a block has no other dim to precondition
 # its Gram along, so its statistics are the plain ones.
@@ -226,10 +232,16 @@ class NativeGroupEngine:
         self._rec = rec
         self._group = group
         self._cfg = cfg
-        self._split = cfg.gemm_mode == "tf32x3"
         self._dist = rec[DISTRIBUTOR]
         self._device = group[PARAMS][0].device
         self._plist = rec[SHAMPOO_PRECONDITIONER_LIST]
+        # Operand format of the step's products at gemm_mode="tf32x3": scaled fp16 pairs (three products at
+        # twice the tf32 rate, half the operand bytes, no larger error) wherever the layouts allow it, tf32
+        # (hi, lo) pairs of fp32 arrays elsewhere.  ``_split`` is the latter; the refreshes use it in both cases.
+        self._refresh_split = cfg.gemm_mode == "tf32x3"
+        self._half = self._refresh_split and self._half_pairs_cover(group, cfg)
+        self._split = self._refresh_split and not self._half
+        self._form = self._ext.HALF_PAIR if self._half else self._split
         self._glist = rec[GRAFTING_PRECONDITIONER_LIST]
         self._packing = group[PRECONDITIONER_CONFIG].use_symmetric_packing
         self._soap = type(group[PRECONDITIONER_CONFIG]) is EigenvalueCorrectedShampooPreconditionerConfig
@@ -311,6 +323,27 @@ class NativeGroupEngine:
     # ------------------------------------------------------------------------------------------
     # Set-up
     # ------------------------------------------------------------------------------------------
+    def _half_pairs_cover(self, group: dict[str, Any], cfg: NativeRuntimeConfig) -> bool:
+        """Half pairs interleave 32 elements along K, which an order-3 block's re-viewed unfoldings keep
+        only if its first two dims are multiples of 32.  Their scale takes a pass over the gradient before
+        the prologue, which a gradient reduced from the peers' memory does not have; the transposing copy
+        of blocks preconditioned on the rows only moves fp32 arrays.  The stand-in of the extension on a CPU
+        has fp32 operands.  Where pairs do apply they win at every size: a step over an 8192 x 8192 weight
+        takes 2.96 ms with them and 4.93 ms with tf32 pairs, one over 1000 x 1337 weights 0.19 and 0.23 ms."""
+        if self._device.type != "cuda":
+            return False
+        if type(group[DISTRIBUTED_CONFIG]) is DDPDistributedConfig and cfg.comm_path == "p2p" and cfg.fuse_gradient_reduction:
+            return False
+        selectors = self._plist._local_preconditioned_dims_selector_list
+        return all(
+            all(sel) and (view.dim() != 3 or (view.shape[0] % 32 == 0 and view.shape[1] % 32 == 0))
+            for view, sel in zip(self._dist.local_blocked_params, selectors, strict=True)
+        )
+
+    def _pad(self, n: int) -> int:
+        """Row pitch of an operand array with ``n`` columns: 16-byte rows, or whole chunks of half pairs."""
+        return (n + 31) // 32 * 32 if self._half else _pad4(n)
+
     def _build_blocks(self) -> None:
         rec, dist = self._rec, self._dist
         dev = self._device
@@ -326,7 +359,12 @@ class NativeGroupEngine:
         moms = rec.get(MOMENTUM_BUFFER_LIST)
         zs = rec.get(WEIGHT_BUFFER_LIST)
         vs = self._glist._local_preconditioner_list if self._graft_kind == _GRAFT_ADAGRAD else None
-        self._norms = torch.zeros(max(len(dist.local_blocked_params), 1), 2, dtype=torch.float32, device=dev)
+        # Zeroed by one fill at the start of a step: the norms, and the meta data of the half-pair operands.
+        count = max(len(dist.local_blocked_params), 1)
+        self._step_scratch = torch.zeros(count * (2 + (_META_SIZE if self._half else 0)), dtype=torch.float32, device=dev)
+        self._norms = self._step_scratch[: 2 * count].view(count, 2)
+        self._meta = self._step_scratch[2 * count :].view(count, _META_SIZE) if self._half else None
+        self._root_meta = torch.zeros(count, 3, 2, dtype=torch.float32, device=dev) if self._half else None
 
         pool = _ZeroPool(dev)
         zeros = pool.zeros
@@ -352,7 +390,7 @@ class NativeGroupEngine:
                 b.view2d = view.view(b.m, b.n)
             else:
                 b.m, b.n = view.shape
-            b.n_pad, b.m_pad = _pad4(b.n), _pad4(b.m)
+            b.n_pad, b.m_pad = self._pad(b.n), self._pad(b.m)
             b.factors = factors_list[i]
             b.m1 = m1s[i] if m1s is not None else None
             b.v = vs[i] if vs is not None else None
@@ -392,14 +430,14 @@ class NativeGroupEngine:
             # Likewise the search direction P [m, n] reuses G (hi part) when the pitches agree.
             b.p = b.g_hi if (b.g_hi is not None and b.n_pad == b.n) else zeros(b.m, b.n)
             dims = tuple(d for d, on in zip((b.m, b.n) if two_d else (b.n,), b.sel, strict=True) if on)
-            b.inv_hi = [zeros(d, _pad4(d)) for d in dims]
-            b.inv_lo = [zeros(d, _pad4(d)) if self._split else None for d in dims]
+            b.inv_hi = [zeros(d, self._pad(d)) for d in dims]
+            b.inv_lo = [zeros(d, self._pad(d)) if self._split else None for d in dims]
             b.ev = b.qt_hi = b.qt_lo = b.t2_hi = b.t2_lo = None
             if self._soap:
                 # inv_hi/inv_lo hold the eigenvector matrices Q_k, qt_* their transposes.
                 b.ev = b.factors.corrected_eigenvalues
-                b.qt_hi = [zeros(d, _pad4(d)) for d in dims]
-                b.qt_lo = [zeros(d, _pad4(d)) if self._split else None for d in dims]
+                b.qt_hi = [zeros(d, self._pad(d)) for d in dims]
+                b.qt_lo = [zeros(d, self._pad(d)) if self._split else None for d in dims]
                 b.t2_hi = zeros(b.n, b.m_pad) if two_d else None
                 b.t2_lo = zeros(b.n, b.m_pad) if two_d and self._split else None
             blocks.append(b)
@@ -417,7 +455,7 @@ class NativeGroupEngine:
         pair = lambda r, cols: (zeros(r, cols), zeros(r, cols) if sp else None)  # noqa: E731
         b.g_hi = b.g_lo = None
         b.gt_hi, b.gt_lo = pair(c, a * bb)
-        b.f_hi, b.f_lo = pair(a * bb, _pad4(c))
+        b.f_hi, b.f_lo = pair(a * bb, self._pad(c))
         b.aux_g_hi, b.aux_g_lo = pair(a, bb * c)
         b.aux_gt_hi, b.aux_gt_lo = pair(bb * c, a)
         # Chain intermediates and the result reuse operand arrays whose last reader (the factor
@@ -427,18 +465,18 @@ class NativeGroupEngine:
         b.d2_lo = b.aux_gt_lo.view(bb, c * a) if sp else None
         b.tt_hi = b.tt_lo = None
         b.p = b.aux_g_hi
-        b.inv_hi = [zeros(d, _pad4(d)) for d in b.dims3]
-        b.inv_lo = [zeros(d, _pad4(d)) if sp else None for d in b.dims3]
+        b.inv_hi = [zeros(d, self._pad(d)) for d in b.dims3]
+        b.inv_lo = [zeros(d, self._pad(d)) if sp else None for d in b.dims3]
         b.ev = b.qt_hi = b.qt_lo = b.t2_hi = b.t2_lo = None
         b.e1_hi = b.e1_lo = b.e2_hi = b.e2_lo = None
         if self._soap:
             # The raw gradient is projected as well (second moment in the eigenbasis): it needs the
             # (ab, c) operand form of G, the transposed eigenvector mirrors, and chain intermediates
             # of its own, since it runs in the same launches as the chain of the filtered gradient.
-            b.g_hi, b.g_lo = pair(a * bb, _pad4(c))
+            b.g_hi, b.g_lo = pair(a * bb, self._pad(c))
             b.ev = b.factors.corrected_eigenvalues
-            b.qt_hi = [zeros(d, _pad4(d)) for d in b.dims3]
-            b.qt_lo = [zeros(d, _pad4(d)) if sp else None for d in b.dims3]
+            b.qt_hi = [zeros(d, self._pad(d)) for d in b.dims3]
+            b.qt_lo = [zeros(d, self._pad(d)) if sp else None for d in b.dims3]
             b.e1_hi, b.e1_lo = pair(c, a * bb)
             b.e2_hi, b.e2_lo = pair(bb, c * a)
 
@@ -524,6 +562,7 @@ class NativeGroupEngine:
                     b.g_hi, b.g_lo, b.gt_hi, b.gt_lo, b.f_hi, b.f_lo, b.p, self._norms[b.index], self._send_ptr(b),
                     self._slot_offset(b), b.ev, 0 if (self._soap or any(b.sel)) else 2,
                 )
+                + ((self._meta[b.index],) if self._half else ())
             )
         for b in blocks:
             if b.dims3 is None:
@@ -533,6 +572,7 @@ class NativeGroupEngine:
             specs.append(
                 (b.param_view.view(a, bb * c), b.grad_offset, b.grad_slot, a, bb * c, bb * c, a)
                 + (None,) * 4 + (b.aux_g_hi, b.aux_g_lo, b.aux_gt_hi, b.aux_gt_lo) + (None,) * 4 + (0, 0, None, 1)
+                + ((self._meta[b.index],) if self._half else ())
             )
         self._table = ext.build_block_table(specs)
         if self._soap:
@@ -548,9 +588,8 @@ class NativeGroupEngine:
             self._build_soap_plans(blocks)
             return
 
-        def op(t: Tensor, rows: int, k: int) -> Tensor:
-            return t[:, :k] if t.shape[1] != k else t
-
+        op = self._operand
+        meta = self._with_meta
         syrk, gemm0, gemm1, gemm2, kl = [], [], [], [], []
         f_transposes = []  # (F hi|lo -> T^T hi|lo) of the blocks preconditioned on the rows only
         pack_flag = F.FLAG_PACKED_C if self._packing else 0
@@ -558,7 +597,7 @@ class NativeGroupEngine:
 
         def chained(a_hi, a_lo, b_hi, b_lo, out_hi, out_lo):
             """Product whose result is only the operand of the next product of the chain."""
-            if sp:
+            if sp or self._half:
                 return (a_hi, a_lo, b_hi, b_lo, None, out_hi, out_lo, None, 0, out_hi.stride(0), F.FLAG_NO_C | F.FLAG_SPLIT_OUT, False)
             return (a_hi, None, b_hi, None, out_hi, None, None, None, out_hi.stride(0), 0, 0, False)
 
@@ -571,14 +610,14 @@ class NativeGroupEngine:
                 xb = (b.aux_gt_hi.view(bb, c * a), lo(b.aux_gt_lo.view(bb, c * a) if sp else None))
                 xc = (b.gt_hi, lo(b.gt_lo))
                 for (x_hi, x_lo), factor, d in ((xa, fm[0], a), (xb, fm[1], bb), (xc, fm[2], c)):
-                    syrk.append((x_hi, x_lo, x_hi, x_lo, factor, None, None, None, d, 0, pack_flag, self._packing))
-                inv = [(b.inv_hi[k][:, :d], lo(b.inv_lo[k][:, :d] if sp else None)) for k, d in enumerate(b.dims3)]
-                f = (b.f_hi[:, :c], lo(b.f_lo[:, :c] if sp else None))
-                gemm0.append(chained(*inv[2], *f, b.d1_hi, b.d1_lo))
+                    syrk.append(meta(b, (x_hi, x_lo, x_hi, x_lo, factor, None, None, None, d, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                inv = [(op(b.inv_hi[k], d, d), op(b.inv_lo[k], d, d) if sp else None) for k, d in enumerate(b.dims3)]
+                f = (op(b.f_hi, a * bb, c), op(b.f_lo, a * bb, c) if sp else None)
+                gemm0.append(meta(b, chained(*inv[2], *f, b.d1_hi, b.d1_lo), "root2", _META_FILTERED, _META_T))
                 d1 = (b.d1_hi.view(c * a, bb), lo(b.d1_lo.view(c * a, bb) if sp else None))
-                gemm1.append(chained(*inv[1], *d1, b.d2_hi, b.d2_lo))
+                gemm1.append(meta(b, chained(*inv[1], *d1, b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
                 d2 = (b.d2_hi.view(bb * c, a), lo(b.d2_lo.view(bb * c, a) if sp else None))
-                gemm2.append((*inv[0], *d2, b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False))
+                gemm2.append(meta(b, (*inv[0], *d2, b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", _META_T2))
                 continue
             two_d = b.order == 2
             left, right = two_d and b.sel[0], b.sel[-1]
@@ -594,18 +633,18 @@ class NativeGroupEngine:
                 a_hi, a_lo = op(b.g_hi, b.m, b.n), (op(b.g_lo, b.m, b.n) if sp else None)
                 ri = (op(b.inv_hi[1], b.n, b.n), op(b.inv_lo[1], b.n, b.n) if sp else None)
                 li = (op(b.inv_hi[0], b.m, b.m), op(b.inv_lo[0], b.m, b.m) if sp else None)
-                kl.append(chained(a_hi, a_lo, *ri, b.y_hi, b.y_lo))
-                kl.append(chained(t_hi, t_lo, *li, b.zt_hi, b.zt_lo))
+                kl.append(meta(b, chained(a_hi, a_lo, *ri, b.y_hi, b.y_lo), _META_GRAD, "root1", _META_U))
+                kl.append(meta(b, chained(t_hi, t_lo, *li, b.zt_hi, b.zt_lo), _META_GRAD, "root0", _META_U2))
                 y = (op(b.y_hi, b.m, b.n), op(b.y_lo, b.m, b.n) if sp else None)
                 zt = (op(b.zt_hi, b.n, b.m), op(b.zt_lo, b.n, b.m) if sp else None)
-                syrk.append((*y, *y, fm[0], None, None, None, b.m, 0, pack_flag, self._packing))
-                syrk.append((*zt, *zt, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing))
+                syrk.append(meta(b, (*y, *y, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_U, _META_U))
+                syrk.append(meta(b, (*zt, *zt, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_U2, _META_U2))
             else:
                 if left:
                     a_hi, a_lo = op(b.g_hi, b.m, b.n), (op(b.g_lo, b.m, b.n) if self._split else None)
-                    syrk.append((a_hi, a_lo, a_hi, a_lo, fm[0], None, None, None, b.m, 0, pack_flag, self._packing))
+                    syrk.append(meta(b, (a_hi, a_lo, a_hi, a_lo, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
                 if right:
-                    syrk.append((t_hi, t_lo, t_hi, t_lo, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing))
+                    syrk.append(meta(b, (t_hi, t_lo, t_hi, t_lo, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
 
             f_hi, f_lo = op(b.f_hi, b.m, b.n), (op(b.f_lo, b.m, b.n) if self._split else None)
             sumsq = self._norms[b.index, 1:2]
@@ -620,17 +659,13 @@ class NativeGroupEngine:
             elif left:
                 r_hi, r_lo = op(b.inv_hi[1], b.n, b.n), (op(b.inv_lo[1], b.n, b.n) if self._split else None)
                 l_hi, l_lo = op(b.inv_hi[0], b.m, b.m), (op(b.inv_lo[0], b.m, b.m) if self._split else None)
-                if self._split:
-                    gemm1.append(
-                        (r_hi, r_lo, f_hi, f_lo, None, b.tt_hi, b.tt_lo, None, 0, b.m_pad, F.FLAG_NO_C | F.FLAG_SPLIT_OUT, False)
-                    )
-                else:
-                    gemm1.append((r_hi, None, f_hi, None, b.tt_hi, None, None, None, b.m_pad, 0, 0, False))
+                gemm1.append(meta(b, chained(r_hi, r_lo, f_hi, f_lo, b.tt_hi, b.tt_lo), "root1", _META_FILTERED, _META_T))
                 tt_hi, tt_lo = op(b.tt_hi, b.n, b.m), (op(b.tt_lo, b.n, b.m) if self._split else None)
-                gemm2.append((l_hi, l_lo, tt_hi, tt_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False))
+                gemm2.append(meta(b, (l_hi, l_lo, tt_hi, tt_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", _META_T))
             else:  # columns only: a 1-D block, or a 2-D block whose rows are not preconditioned
                 r_hi, r_lo = op(b.inv_hi[-1], b.n, b.n), (op(b.inv_lo[-1], b.n, b.n) if self._split else None)
-                gemm2.append((f_hi, f_lo, r_hi, r_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False))
+                root = f"root{len(b.inv_hi) - 1}"
+                gemm2.append(meta(b, (f_hi, f_lo, r_hi, r_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), _META_FILTERED, root))
         self._f_transpose_table = ext.build_transpose_table(f_transposes) if f_transposes else None
         # the pushing plan pairs one final product with every block (see the rule at _gemm_push)
         assert not self._gemm_push or len(gemm2) == len(blocks)
@@ -643,10 +678,25 @@ class NativeGroupEngine:
             # Same products; the result goes to the block's slot of every gather buffer instead of b.p.
             flags = F.FLAG_SUMSQ | F.FLAG_NO_C | F.FLAG_PEER_PUSH
             push = [
-                (s[0], s[1], s[2], s[3], None, None, None, s[7], s[8], 0, flags, False, self._slot_offset(b))
+                (s[0], s[1], s[2], s[3], None, None, None, s[7], s[8], 0, flags, False, self._slot_offset(b), *s[13:])
                 for s, b in zip(gemm2, blocks, strict=True)
             ]
             self._gemm2_push_plan = ext.build_gemm_plan(push)
+
+    def _operand(self, t: Tensor, rows: int, k: int) -> Tensor:
+        """The K extent of an operand array the products read (half pairs: whole chunks, zero padded)."""
+        return t[:, :k] if t.shape[1] != k and not self._half else t
+
+    def _with_meta(self, b: _Block, spec: tuple, a_slot: int | str, b_slot: int | str, d_slot: int | None = None) -> tuple:
+        """``spec`` with the meta data of its half-pair operands and split output: slots of the block's step
+        scratch, or ``"root<k>"`` for the mirror of its k-th inverse root (or eigenbasis, or its transpose)."""
+        if not self._half:
+            return spec
+
+        def of(slot):
+            return self._root_meta[b.index, int(slot[4:])] if isinstance(slot, str) else self._meta[b.index, slot : slot + 2]
+
+        return (*spec, None, None, (of(a_slot), of(b_slot), None if d_slot is None else of(d_slot)))
 
     def _build_soap_plans(self, blocks: list[_Block]) -> None:
         """GEMM plans of the eigenvalue-corrected step.  With Qt the transposed eigenvector
@@ -660,12 +710,14 @@ class NativeGroupEngine:
         ext, split = self._ext, self._split
         F = ext
 
+        meta = self._with_meta
+
         def pair(hi: Tensor, lo: Tensor | None, k: int) -> tuple[Tensor, Tensor | None]:
-            return hi[:, :k], (lo[:, :k] if lo is not None else None)
+            return self._operand(hi, 0, k), (lo[:, :k] if lo is not None else None)
 
         def chained(a, b, out_hi, out_lo):
             """Product whose result is only an operand of the next product."""
-            if split:
+            if split or self._half:
                 return (*_ab(a, b), None, out_hi, out_lo, None, 0, out_hi.stride(0), F.FLAG_NO_C | F.FLAG_SPLIT_OUT, False)
             return (*_ab(a, b), out_hi, None, None, None, out_hi.stride(0), 0, 0, False)
 
@@ -687,7 +739,7 @@ class NativeGroupEngine:
                 xb = (b.aux_gt_hi.view(bb, c * a), lo(b.aux_gt_lo.view(bb, c * a) if split else None))
                 xc = (b.gt_hi, lo(b.gt_lo))
                 for x, factor, d in ((xa, fm[0], a), (xb, fm[1], bb), (xc, fm[2], c)):
-                    syrk.append((*_ab(x, x), factor, None, None, None, d, 0, pack_flag, self._packing))
+                    syrk.append(meta(b, (*_ab(x, x), factor, None, None, None, d, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
                 q = [pair(b.inv_hi[k], b.inv_lo[k], d) for k, d in enumerate(b.dims3)]
                 qt = [pair(b.qt_hi[k], b.qt_lo[k], d) for k, d in enumerate(b.dims3)]
                 g3, f3 = pair(b.g_hi, b.g_lo, c), pair(b.f_hi, b.f_lo, c)
@@ -695,16 +747,16 @@ class NativeGroupEngine:
                 def as_rows(hi, lo_, rows, cols):
                     return (hi.view(rows, cols), lo_.view(rows, cols) if lo_ is not None else None)
 
-                st_a0.append(chained(qt[2], g3, b.e1_hi, b.e1_lo))
-                st_a0.append(chained(qt[2], f3, b.d1_hi, b.d1_lo))
-                st_a.append(chained(qt[1], as_rows(b.e1_hi, b.e1_lo, c * a, bb), b.e2_hi, b.e2_lo))
-                st_a.append(chained(qt[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo))
+                st_a0.append(meta(b, chained(qt[2], g3, b.e1_hi, b.e1_lo), "root2", _META_GRAD, _META_U))
+                st_a0.append(meta(b, chained(qt[2], f3, b.d1_hi, b.d1_lo), "root2", _META_FILTERED, _META_T))
+                st_a.append(meta(b, chained(qt[1], as_rows(b.e1_hi, b.e1_lo, c * a, bb), b.e2_hi, b.e2_lo), "root1", _META_U, _META_U2))
+                st_a.append(meta(b, chained(qt[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
                 ev = b.ev.view(a, bb * c)
-                st_v.append((*_ab(qt[0], as_rows(b.e2_hi, b.e2_lo, bb * c, a)), ev, None, None, None, bb * c, 0, F.FLAG_SQUARE_ACC, False))
-                st_f.append((*_ab(qt[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, None, bb * c, 0, 0, False))
-                st_u0.append(chained(q[2], f3, b.d1_hi, b.d1_lo))
-                st_u1.append(chained(q[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo))
-                st_u2.append((*_ab(q[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False))
+                st_v.append(meta(b, (*_ab(qt[0], as_rows(b.e2_hi, b.e2_lo, bb * c, a)), ev, None, None, None, bb * c, 0, F.FLAG_SQUARE_ACC, False), "root0", _META_U2))
+                st_f.append(meta(b, (*_ab(qt[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, None, bb * c, 0, 0, False), "root0", _META_T2))
+                st_u0.append(meta(b, chained(q[2], f3, b.d1_hi, b.d1_lo), "root2", _META_SCALED, _META_T))
+                st_u1.append(meta(b, chained(q[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
+                st_u2.append(meta(b, (*_ab(q[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", _META_T2))
                 continue
             two_d = b.order == 2
             g = pair(b.g_hi, b.g_lo, b.n)
@@ -712,23 +764,23 @@ class NativeGroupEngine:
             f = pair(b.f_hi, b.f_lo, b.n)
             sumsq = self._norms[b.index, 1:2]
             if two_d:
-                syrk.append((*_ab(g, g), fm[0], None, None, None, b.m, 0, pack_flag, self._packing))
-            syrk.append((*_ab(gt, gt), fm[-1], None, None, None, b.n, 0, pack_flag, self._packing))
+                syrk.append(meta(b, (*_ab(g, g), fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+            syrk.append(meta(b, (*_ab(gt, gt), fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
             r = 1 if two_d else 0
             qr, qrt = pair(b.inv_hi[r], b.inv_lo[r], b.n), pair(b.qt_hi[r], b.qt_lo[r], b.n)
             if two_d:
                 ql, qlt = pair(b.inv_hi[0], b.inv_lo[0], b.m), pair(b.qt_hi[0], b.qt_lo[0], b.m)
                 t2, tt = pair(b.t2_hi, b.t2_lo, b.m), pair(b.tt_hi, b.tt_lo, b.m)
-                st_a.append(chained(qrt, g, b.t2_hi, b.t2_lo))
-                st_a.append(chained(qrt, f, b.tt_hi, b.tt_lo))
-                st_v.append((*_ab(qlt, t2), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False))
-                st_f.append((*_ab(qlt, tt), b.p, None, None, None, b.n, 0, 0, False))
-                st_u1.append(chained(qr, f, b.tt_hi, b.tt_lo))
-                st_u2.append((*_ab(ql, tt), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False))
+                st_a.append(meta(b, chained(qrt, g, b.t2_hi, b.t2_lo), "root1", _META_GRAD, _META_U))
+                st_a.append(meta(b, chained(qrt, f, b.tt_hi, b.tt_lo), "root1", _META_FILTERED, _META_T))
+                st_v.append(meta(b, (*_ab(qlt, t2), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), "root0", _META_U))
+                st_f.append(meta(b, (*_ab(qlt, tt), b.p, None, None, None, b.n, 0, 0, False), "root0", _META_T))
+                st_u1.append(meta(b, chained(qr, f, b.tt_hi, b.tt_lo), "root1", _META_SCALED, _META_T))
+                st_u2.append(meta(b, (*_ab(ql, tt), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", _META_T))
             else:
-                st_v.append((*_ab(g, qrt), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False))
-                st_f.append((*_ab(f, qrt), b.p, None, None, None, b.n, 0, 0, False))
-                st_u2.append((*_ab(f, qr), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False))
+                st_v.append(meta(b, (*_ab(g, qrt), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), _META_GRAD, "root0"))
+                st_f.append(meta(b, (*_ab(f, qrt), b.p, None, None, None, b.n, 0, 0, False), _META_FILTERED, "root0"))
+                st_u2.append(meta(b, (*_ab(f, qr), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), _META_SCALED, "root0"))
         self._syrk_plan = ext.build_gemm_plan(syrk)
         mk = lambda specs: ext.build_gemm_plan(specs) if specs else None  # noqa: E731
         self._soap_plans = {
@@ -743,6 +795,9 @@ class NativeGroupEngine:
         ext, sp = self._ext, self._split
         todo = self._blocks if blocks is None else blocks
         if not todo:
+            return
+        if self._half:
+            self._refresh_pair_mirrors(todo)
             return
         if self._soap:
             plain, transposed = [], []
@@ -760,27 +815,58 @@ class NativeGroupEngine:
             return
         specs = []
         for b in todo:
-            if self._eigdec:
-                from fractions import Fraction
-
-                from optimizers_b200.matrix import functions as mf
-
-                kf = b.factors
-                stability = kf.amortized_computation_config.rank_deficient_stability_config
-                sources = [
-                    mf.matrix_inverse_root_from_eigendecomposition(
-                        L=lam, Q=Q, root=Fraction(root), epsilon=kf.epsilon, rank_deficient_stability_config=stability
-                    ).contiguous()
-                    for Q, lam, root in zip(kf.factor_matrices_eigenvectors, kf.factor_matrices_eigenvalues, kf.roots, strict=True)
-                ]
-            else:
-                # the state itself: the packed upper triangle or the full matrix
-                sources = [m if m.dim() == 1 or m.stride(-1) == 1 else m.contiguous() for m in b.factors.inv_factor_matrices]
+            sources = self._root_sources(b)
             for k, src in enumerate(sources):
                 d = b.inv_hi[k].shape[0]
                 specs.append((src, d, b.inv_hi[k][:, :d], b.inv_lo[k][:, :d] if sp else None))
         if specs:
             ext.unpack_split(*ext.build_unpack_table(specs))
+
+    def _root_sources(self, b: _Block) -> list[Tensor]:
+        """The inverse roots of a block as its state holds them (packed upper triangles or full matrices)."""
+        if self._eigdec:
+            from fractions import Fraction
+
+            from optimizers_b200.matrix import functions as mf
+
+            kf = b.factors
+            stability = kf.amortized_computation_config.rank_deficient_stability_config
+            return [
+                mf.matrix_inverse_root_from_eigendecomposition(
+                    L=lam, Q=Q, root=Fraction(root), epsilon=kf.epsilon, rank_deficient_stability_config=stability
+                ).contiguous()
+                for Q, lam, root in zip(kf.factor_matrices_eigenvectors, kf.factor_matrices_eigenvalues, kf.roots, strict=True)
+            ]
+        return [m if m.dim() == 1 or m.stride(-1) == 1 else m.contiguous() for m in b.factors.inv_factor_matrices]
+
+    def _refresh_pair_mirrors(self, todo: list[_Block]) -> None:
+        """Half-pair mirrors from the state: the full fp32 matrices are unpacked into the mirrors' own
+        memory and converted there."""
+        ext = self._ext
+        unpack, fresh = [], []
+        for b in todo:
+            if self._soap:
+                sources = [Q if Q.stride(-1) == 1 else Q.contiguous() for Q in b.factors.factor_matrices_eigenvectors]
+            else:
+                sources = self._root_sources(b)
+            for k, src in enumerate(sources):
+                d = b.inv_hi[k].shape[0]
+                unpack.append((src, d, b.inv_hi[k][:, :d], None))
+                fresh.append((b, k))
+        if unpack:
+            ext.unpack_split(*ext.build_unpack_table(unpack))
+            self._convert_pair_mirrors(fresh)
+
+    def _convert_pair_mirrors(self, fresh: list[tuple[_Block, int]]) -> None:
+        """Measures the fp32 matrices that stand in the mirrors ``(block, k)`` for their scale and turns them into
+        half pairs in place; eigenbases also into their transposes."""
+        ext = self._ext
+        metas = [self._root_meta[b.index, k] for b, k in fresh]
+        torch._foreach_zero_(metas)
+        ext.pair_mirrors(*ext.build_pair_table([
+            (b.inv_hi[k][:, : b.inv_hi[k].shape[0]], b.inv_hi[k], b.qt_hi[k] if self._soap else None, m)
+            for (b, k), m in zip(fresh, metas, strict=True)
+        ]))
 
     # ------------------------------------------------------------------------------------------
     # Hooks called by the optimizer
@@ -1006,35 +1092,41 @@ class NativeGroupEngine:
             g_bc2 = float(glist._bias_correction2)
         l2 = weight_decay if (weight_decay_type == WeightDecayType.L2) else 0.0
 
-        self._norms.zero_()
+        self._step_scratch.zero_()
         blocks_t, tiles_t, n_tiles = self._table
         ext.grad_prologue(
             blocks_t, tiles_t, n_tiles, self._grad_ptrs_dev, l2, beta1, beta3, bc1, self._graft_kind,
-            g_beta2, g_weight, g_bc2, g_eps, self._split, self._status,
+            g_beta2, g_weight, g_bc2, g_eps, self._form, self._status,
             self._arena.world if self._pull else 0, 1.0 / self._arena.world if self._pull else 1.0,
+            *((graft_only,) if self._half else ()),
         )
-        launches += 2
+        launches += 3 if self._half else 2
         self._mark("grad_prologue")
         if not self._soap and self._kl_plan is not None:
-            ext.run_gemm_plan(*self._kl_plan, 1.0, 0.0, self._split, self._status)
+            ext.run_gemm_plan(*self._kl_plan, 1.0, 0.0, self._form, self._status)
             launches += 1
         if self._syrk_plan is not None:
-            ext.run_gemm_plan(*self._syrk_plan, plist._weighting_factor, plist._beta2, self._split, self._status)
+            ext.run_gemm_plan(*self._syrk_plan, plist._weighting_factor, plist._beta2, self._form, self._status)
             launches += 1
         self._mark("factor_syrk")
 
         if refresh:
-            self._refresh(self._active_blocks)
+            try:
+                self._refresh(self._active_blocks)
+            except Exception:
+                if self._half:  # a refresh that raised may have left fp32 matrices in the mirrors
+                    self.refresh_inverse_mirrors(self._active_blocks)
+                raise
             self._mark("refresh")
 
         if self._soap:
             launches += self._soap_step(plist, graft_only)
         elif not graft_only:
             if self._gemm0_plan is not None:
-                ext.run_gemm_plan(*self._gemm0_plan, 1.0, 0.0, self._split, self._status)
+                ext.run_gemm_plan(*self._gemm0_plan, 1.0, 0.0, self._form, self._status)
                 launches += 1
             if self._gemm1_plan is not None:
-                ext.run_gemm_plan(*self._gemm1_plan, 1.0, 0.0, self._split, self._status)
+                ext.run_gemm_plan(*self._gemm1_plan, 1.0, 0.0, self._form, self._status)
                 launches += 1
             if self._f_transpose_table is not None:
                 ext.transpose_split(*self._f_transpose_table)
@@ -1042,10 +1134,10 @@ class NativeGroupEngine:
             if use_push:
                 # The last preconditioner GEMM stores its tiles into every rank's gather buffer.
                 ext.run_gemm_plan_push(
-                    *self._gemm2_push_plan, 1.0, 0.0, self._split, self._status, self._gather_bases, self._comm_dtype_code
+                    *self._gemm2_push_plan, 1.0, 0.0, self._form, self._status, self._gather_bases, self._comm_dtype_code
                 )
             elif self._gemm2_plan is not None:
-                ext.run_gemm_plan(*self._gemm2_plan, 1.0, 0.0, self._split, self._status)
+                ext.run_gemm_plan(*self._gemm2_plan, 1.0, 0.0, self._form, self._status)
             launches += 1
 
         self._mark("preconditioner_gemms")
@@ -1071,8 +1163,9 @@ class NativeGroupEngine:
 
     def _soap_step(self, plist: Any, graft_only: bool) -> int:
         """Second-moment update in the eigenbasis (every step) and, unless only the grafting
-        direction is needed, project -> scale -> unproject of the filtered gradient."""
-        ext, plans, split = self._ext, self._soap_plans, self._split
+        direction is needed, project -> scale -> unproject of the filtered gradient (whose projection
+        runs in the first stages either way: a step that only takes the grafting direction leaves it unread)."""
+        ext, plans, split = self._ext, self._soap_plans, self._form
         run = lambda key, alpha=1.0, beta=0.0: ext.run_gemm_plan(*plans[key], alpha, beta, split, self._status)  # noqa: E731
         launches = 0
         for stage in ("a0", "a"):  # first stages of the projections: order-3 blocks only, then 2-D and order-3
@@ -1091,7 +1184,7 @@ class NativeGroupEngine:
                 run(stage)
                 launches += 1
         run("u2")
-        return launches + 2 + len(self._eig_tables)
+        return launches + 2 + len(self._eig_tables) * (2 if self._half else 1)
 
     def _refresh(self, blocks: list[_Block]) -> None:
         """Amortised computation for the given blocks: batched native path for the eigen root
@@ -1111,15 +1204,17 @@ class NativeGroupEngine:
                     b.factors.amortized_computation(bias_correction2=plist._bias_correction2)
         elif self._eigdec:
             if batched.eigdec_refresh_supported(cfg):
-                batched.batched_eigen_refresh(self._ext, blocks, plist._bias_correction2, self._split, self._status)
+                fresh = batched.batched_eigen_refresh(self._ext, blocks, plist._bias_correction2, self._refresh_split, self._status)
+                if self._half and fresh:
+                    self._convert_pair_mirrors(fresh)
                 self.check_status()
                 return  # the mirrors were written by the refresh itself
             for b in blocks:
                 b.factors.amortized_computation(bias_correction2=plist._bias_correction2)
         elif batched.eigen_refresh_supported(cfg):
-            batched.batched_eigen_refresh(self._ext, blocks, plist._bias_correction2, self._split, self._status)
+            batched.batched_eigen_refresh(self._ext, blocks, plist._bias_correction2, self._refresh_split, self._status)
         elif batched.newton_refresh_supported(cfg):
-            batched.batched_newton_refresh(self._ext, blocks, plist._bias_correction2, self._split, self._status)
+            batched.batched_newton_refresh(self._ext, blocks, plist._bias_correction2, self._refresh_split, self._status)
         else:
             for b in blocks:
                 b.factors.amortized_computation(bias_correction2=plist._bias_correction2)

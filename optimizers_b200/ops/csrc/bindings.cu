@@ -174,6 +174,9 @@ class PlanBuilder {
     float* d_hi = nullptr;
     float* d_lo = nullptr;
     float* sumsq = nullptr;
+    const float* a_meta = nullptr;  // half pairs: PairMeta of both operands and of the split output
+    const float* b_meta = nullptr;
+    float* d_meta = nullptr;
     int M = 0, N = 0, K = 0, ldc = 0, ldd = 0, flags = 0;
     long long push_offset = 0;
     bool upper_tiles_only = false;
@@ -217,7 +220,26 @@ class PlanBuilder {
                   "mirrored output needs a square, unpacked upper-tile problem");
     }
     if (!(p.flags & kFlagNoC)) TORCH_CHECK(p.c != nullptr, "C is required unless kFlagNoC is set");
-    if (p.flags & kFlagSplitOut) TORCH_CHECK(p.d_hi != nullptr && p.d_lo != nullptr, "split output needs d_hi and d_lo");
+    p.a_meta = q.a_meta;
+    p.b_meta = q.b_meta;
+    p.d_meta = q.d_meta;
+    const bool half = p.a_meta != nullptr;
+    TORCH_CHECK(problems_.empty() || half == half_, "a plan holds one operand format");
+    half_ = half;
+    if (half) {
+      TORCH_CHECK(p.b_meta != nullptr, "both operands of a half-pair product need their meta data");
+      TORCH_CHECK(q.K % kBK == 0, "half-pair operands are padded to a multiple of ", kBK, " along K");
+      TORCH_CHECK(!(p.flags & kFlagMirror), "mirrored output has no half-pair form");
+      if (p.flags & kFlagSplitOut) {
+        TORCH_CHECK((p.flags & kFlagNoC) && !(p.flags & (kFlagSumSq | kFlagTrace | kFlagAddDiag | kFlagPackedC)),
+                    "a half-pair split output stands alone");
+        TORCH_CHECK(p.d_hi != nullptr && p.d_meta != nullptr && p.ldd % kBK == 0 && p.ldd >= p.N &&
+                        reinterpret_cast<uintptr_t>(p.d_hi) % 16 == 0,
+                    "a half-pair split output needs its meta data, a 16-byte aligned base and a pitch that is a multiple of ", kBK);
+      }
+    } else if (p.flags & kFlagSplitOut) {
+      TORCH_CHECK(p.d_hi != nullptr && p.d_lo != nullptr, "split output needs d_hi and d_lo");
+    }
     if (p.flags & (kFlagSumSq | kFlagTrace)) TORCH_CHECK(p.sumsq != nullptr, "sumsq output missing");
     problems_.push_back(p);
     upper_.push_back(q.upper_tiles_only);
@@ -243,15 +265,46 @@ class PlanBuilder {
       const int v = env != nullptr ? std::atoi(env) : 12;
       return v > 0 ? v : 12;
     }();
+    // Half pairs run 128 x 128 or 128 x 256 tiles.  A wide tile takes 1.45 times as long as a narrow one
+    // for twice the work (its B operand is read from shared memory once for twice the rows), but
+    // halves the number of tiles: the width with the lower estimated time per launch is taken.
+    int widest = kBN;
+    if (half_) {
+      const int sms = at::cuda::getDeviceProperties(device_.index())->multiProcessorCount;
+      int64_t narrow = 0, wide = 0;
+      for (const Order& o : order) {
+        const GemmProblem& p = problems_[o.problem];
+        for (int m0 = 0; m0 < p.M; m0 += kBM) {
+          const int cols = (p.N - (upper_[o.problem] ? m0 : 0) + kBN - 1) / kBN;
+          narrow += cols;
+          wide += (cols + 1) / 2;
+        }
+      }
+      if (1.45 * static_cast<double>((wide + sms - 1) / sms) < static_cast<double>((narrow + sms - 1) / sms)) widest = 2 * kBN;
+    }
     for (const Order& o : order) {
       const GemmProblem& p = problems_[o.problem];
       const bool upper = upper_[o.problem];
+      if (widest > kBN) {
+        // Row tiles of an upper-triangle problem start at their own diagonal, so the columns of a band
+        // are walked in steps from there.
+        for (int band = 0; band < p.M; band += kBandRows * kBM) {
+          const int band_end = std::min(p.M, band + kBandRows * kBM);
+          for (int step = 0; (upper ? band : 0) + step < p.N; step += widest) {
+            for (int m0 = band; m0 < band_end; m0 += kBM) {
+              const int n0 = (upper ? m0 : 0) + step;
+              if (n0 < p.N) tiles_.push_back({o.problem, m0, n0, p.N - n0 > kBN ? widest : kBN});
+            }
+          }
+        }
+        continue;
+      }
       for (int band = 0; band < p.M; band += kBandRows * kBM) {
         const int band_end = std::min(p.M, band + kBandRows * kBM);
         for (int n0 = upper ? band : 0; n0 < p.N; n0 += kBN) {
           for (int m0 = band; m0 < band_end; m0 += kBM) {
             if (upper && n0 < m0) continue;
-            tiles_.push_back({o.problem, m0, n0, 0});
+            tiles_.push_back({o.problem, m0, n0, kBN});
           }
         }
       }
@@ -284,7 +337,8 @@ class PlanBuilder {
     std::memcpy(static_cast<uint8_t*>(host.data_ptr()) + table_bytes, maps_.data(), map_bytes);
     buffer.copy_(host, /*non_blocking=*/true);
     auto d_tiles = upload_bytes(tiles_.data(), tiles_.size() * sizeof(GemmTile), device_);
-    return {buffer, d_tiles};
+    // The element type of the tile list tells a half-pair plan from an fp32 one (gemm_mode below).
+    return {buffer, half_ ? d_tiles.view(torch::kInt32) : d_tiles};
   }
 
  private:
@@ -306,7 +360,15 @@ class PlanBuilder {
   std::map<std::array<int64_t, 5>, int> cache_;
   torch::Device device_{torch::kCPU};
   int launch_begin_ = 0;
+  bool half_ = false;
 };
+
+// `mode` as a GemmMode, checked against the operand format the plan was built for.
+GemmMode gemm_mode(int64_t mode, const torch::Tensor& tiles) {
+  TORCH_CHECK(mode >= kGemmTf32 && mode <= kGemmHalfPair, "unknown GEMM mode ", mode);
+  TORCH_CHECK((mode == kGemmHalfPair) == (tiles.scalar_type() == torch::kInt32), "GEMM mode and operand format of the plan differ");
+  return static_cast<GemmMode>(mode);
+}
 
 // Holds the tensors of one Python GEMM spec alive while the builder refers to them.
 struct SpecTensors {
@@ -315,10 +377,12 @@ struct SpecTensors {
 };
 
 // Spec fields: (a_hi, a_lo | None, b_hi, b_lo | None, c | None, d_hi | None, d_lo | None, sumsq | None,
-//               ldc, ldd, flags, upper_tiles_only [, push_offset [, (a_row0, a_k0, b_row0, b_k0, M, N, K)]])
-// With the last field the operands are views, of the given origin and extent, of the arrays passed.
+//               ldc, ldd, flags, upper_tiles_only [, push_offset [, (a_row0, a_k0, b_row0, b_k0, M, N, K)
+//               [, (a_meta, b_meta, d_meta | None)]]])
+// With a view field the operands are views, of the given origin and extent, of the arrays passed.  With the last
+// field the operands and the split output are half pairs (a_lo, b_lo and d_lo are None).
 void add_spec(PlanBuilder& builder, const py::tuple& s, std::vector<std::unique_ptr<SpecTensors>>& keep) {
-  TORCH_CHECK(s.size() >= 12 && s.size() <= 14, "GEMM spec must have 12 to 14 fields");
+  TORCH_CHECK(s.size() >= 12 && s.size() <= 15, "GEMM spec must have 12 to 15 fields");
   keep.push_back(std::make_unique<SpecTensors>());
   SpecTensors& g = *keep.back();
   g.a_hi = s[0].cast<torch::Tensor>();
@@ -345,7 +409,7 @@ void add_spec(PlanBuilder& builder, const py::tuple& s, std::vector<std::unique_
   q.push_offset = s.size() >= 13 && !s[12].is_none() ? s[12].cast<int64_t>() : 0;
   if (q.flags & kFlagPeerPush) TORCH_CHECK(s.size() >= 13 && !s[12].is_none(), "a pushing problem needs its slot offset");
   if (q.flags & kFlagTrace) TORCH_CHECK(g.sumsq.has_value() && g.sumsq->numel() >= 2, "trace output needs a two-element sumsq");
-  if (s.size() == 14 && !s[13].is_none()) {
+  if (s.size() >= 14 && !s[13].is_none()) {
     const auto view = s[13].cast<std::vector<int64_t>>();
     TORCH_CHECK(view.size() == 7, "operand view must be (a_row0, a_k0, b_row0, b_k0, M, N, K)");
     q.a.row0 = static_cast<int>(view[0]);
@@ -360,6 +424,13 @@ void add_spec(PlanBuilder& builder, const py::tuple& s, std::vector<std::unique_
     q.N = static_cast<int>(g.b_hi.size(0));
     q.K = static_cast<int>(g.a_hi.size(1));
     TORCH_CHECK(g.b_hi.size(1) == q.K, "A and B must agree on K");
+  }
+  if (s.size() == 15 && !s[14].is_none()) {
+    const auto metas = s[14].cast<std::tuple<torch::Tensor, torch::Tensor, std::optional<torch::Tensor>>>();
+    for (const torch::Tensor* t : {&std::get<0>(metas), &std::get<1>(metas)}) TORCH_CHECK(t->numel() >= 2, "meta data has two entries");
+    q.a_meta = fptr(std::get<0>(metas));
+    q.b_meta = fptr(std::get<1>(metas));
+    q.d_meta = fptr(std::get<2>(metas));
   }
   builder.add(q);
 }
@@ -393,33 +464,33 @@ std::tuple<torch::Tensor, torch::Tensor, std::vector<std::pair<int64_t, int64_t>
 }
 
 void run_gemm_range(const torch::Tensor& problems, const torch::Tensor& tiles, int64_t first_tile, int64_t num_tiles,
-                    double alpha, double beta, bool split, torch::Tensor status, double gamma) {
+                    double alpha, double beta, int64_t split, torch::Tensor status, double gamma) {
   LaunchScope scope("ob200::grouped_gemm");
   if (num_tiles <= 0) return;
   c10::cuda::CUDAGuard guard(problems.device());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   launch_grouped_gemm(reinterpret_cast<const GemmProblem*>(problems.data_ptr()),
                       reinterpret_cast<const GemmTile*>(tiles.data_ptr()) + first_tile, static_cast<int>(num_tiles),
-                      static_cast<float>(alpha), static_cast<float>(beta), split, status.data_ptr<int>(), sms,
+                      static_cast<float>(alpha), static_cast<float>(beta), gemm_mode(split, tiles), status.data_ptr<int>(), sms,
                       at::cuda::getCurrentCUDAStream(), nullptr, static_cast<float>(gamma));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
 void run_gemm_plan(const torch::Tensor& problems, const torch::Tensor& tiles, int64_t num_tiles, double alpha,
-                   double beta, bool split, torch::Tensor status, double gamma) {
+                   double beta, int64_t split, torch::Tensor status, double gamma) {
   LaunchScope scope("ob200::grouped_gemm");
   c10::cuda::CUDAGuard guard(problems.device());
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   launch_grouped_gemm(reinterpret_cast<const GemmProblem*>(problems.data_ptr()),
                       reinterpret_cast<const GemmTile*>(tiles.data_ptr()), static_cast<int>(num_tiles),
-                      static_cast<float>(alpha), static_cast<float>(beta), split, status.data_ptr<int>(), sms,
+                      static_cast<float>(alpha), static_cast<float>(beta), gemm_mode(split, tiles), status.data_ptr<int>(), sms,
                       at::cuda::getCurrentCUDAStream(), nullptr, static_cast<float>(gamma));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
 // run_gemm_plan with the kFlagPeerPush problems storing into the gather buffers at `peer_bases`.
 void run_gemm_plan_push(const torch::Tensor& problems, const torch::Tensor& tiles, int64_t num_tiles, double alpha,
-                        double beta, bool split, torch::Tensor status, const std::vector<int64_t>& peer_bases,
+                        double beta, int64_t split, torch::Tensor status, const std::vector<int64_t>& peer_bases,
                         int64_t send_dtype) {
   LaunchScope scope("ob200::grouped_gemm_push");
   c10::cuda::CUDAGuard guard(problems.device());
@@ -431,20 +502,20 @@ void run_gemm_plan_push(const torch::Tensor& problems, const torch::Tensor& tile
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   launch_grouped_gemm(reinterpret_cast<const GemmProblem*>(problems.data_ptr()),
                       reinterpret_cast<const GemmTile*>(tiles.data_ptr()), static_cast<int>(num_tiles),
-                      static_cast<float>(alpha), static_cast<float>(beta), split, status.data_ptr<int>(), sms,
+                      static_cast<float>(alpha), static_cast<float>(beta), gemm_mode(split, tiles), status.data_ptr<int>(), sms,
                       at::cuda::getCurrentCUDAStream(), &push);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
 // Block table.  Each spec: (param_view, grad_offset, grad_slot, m, n, n_pad, m_pad, m1, v, mom, z,
-//                           g_hi, g_lo, gt_hi, gt_lo, f_hi, f_lo, p, norms, send_ptr, slot_offset, ev)
+//                           g_hi, g_lo, gt_hi, gt_lo, f_hi, f_lo, p, norms, send_ptr, slot_offset, ev, aux [, meta])
 std::tuple<torch::Tensor, torch::Tensor, int64_t> build_block_table(const std::vector<py::tuple>& specs) {
   std::vector<BlockDesc> blocks(specs.size());
   std::vector<TileRef> tiles;
   torch::Device device(torch::kCPU);
   for (size_t i = 0; i < specs.size(); ++i) {
     const py::tuple& s = specs[i];
-    TORCH_CHECK(s.size() == 23, "block spec must have 23 fields");
+    TORCH_CHECK(s.size() == 23 || s.size() == 24, "block spec must have 23 or 24 fields");
     BlockDesc& b = blocks[i];
     std::memset(&b, 0, sizeof(b));
     auto param = s[0].cast<torch::Tensor>();
@@ -481,6 +552,12 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t> build_block_table(const std::v
     b.slot_offset = s[20].cast<int64_t>();
     b.ev = opt(21);
     b.aux = s[22].cast<int>();
+    if (s.size() == 24) {
+      const auto meta = s[23].cast<torch::Tensor>();
+      TORCH_CHECK(meta.numel() >= 6 && meta.is_contiguous(), "block meta data has six entries");
+      b.meta = meta.data_ptr<float>();
+      TORCH_CHECK(b.n_pad % kBK == 0 && b.m_pad % kBK == 0, "half-pair arrays have pitches that are multiples of ", kBK);
+    }
   }
   // Tiles of 32 rows x 128 columns.
   for (size_t i = 0; i < specs.size(); ++i) {
@@ -499,8 +576,8 @@ inline const TileRef* tile_ptr(const torch::Tensor& tiles) { return reinterpret_
 void grad_prologue(const torch::Tensor& blocks, const torch::Tensor& tiles, int64_t num_tiles,
                    const torch::Tensor& grad_ptrs, double l2_weight_decay, double beta1, double beta3,
                    double bias_correction1, int64_t graft_kind, double graft_beta2, double graft_weight,
-                   double graft_bc2, double graft_eps, bool write_split, torch::Tensor status,
-                   int64_t num_grad_peers, double grad_scale) {
+                   double graft_bc2, double graft_eps, int64_t write_split, torch::Tensor status,
+                   int64_t num_grad_peers, double grad_scale, bool filtered_plain) {
   LaunchScope scope("ob200::grad_prologue");
   c10::cuda::CUDAGuard guard(blocks.device());
   PrologueArgs a;
@@ -517,7 +594,10 @@ void grad_prologue(const torch::Tensor& blocks, const torch::Tensor& tiles, int6
   a.graft_weight = static_cast<float>(graft_weight);
   a.graft_bias_correction2 = static_cast<float>(graft_bc2);
   a.graft_epsilon = static_cast<float>(graft_eps);
-  a.write_split = write_split ? 1 : 0;
+  TORCH_CHECK(write_split >= kFormPlain && write_split <= kFormPair, "unknown operand form ", write_split);
+  TORCH_CHECK(write_split != kFormPair || num_grad_peers == 0, "half pairs need the gradient in local memory");
+  a.form = static_cast<int>(write_split);
+  a.filtered_plain = filtered_plain ? 1 : 0;
   a.status = status.data_ptr<int>();
   a.num_grad_peers = static_cast<int>(num_grad_peers);
   a.grad_scale = static_cast<float>(grad_scale);
@@ -584,12 +664,12 @@ void gathered_apply_scaled(const torch::Tensor& blocks, const torch::Tensor& til
 }
 
 void eig_scale(const torch::Tensor& blocks, const torch::Tensor& tiles, int64_t num_tiles, double bc2, double inv_root,
-               double eps, bool write_split) {
+               double eps, int64_t write_split) {
   LaunchScope scope("ob200::eig_scale");
   c10::cuda::CUDAGuard guard(blocks.device());
   launch_eig_scale(reinterpret_cast<const BlockDesc*>(blocks.data_ptr()), tile_ptr(tiles),
                    static_cast<int>(num_tiles), static_cast<float>(bc2), static_cast<float>(inv_root),
-                   static_cast<float>(eps), write_split ? 1 : 0, at::cuda::getCurrentCUDAStream());
+                   static_cast<float>(eps), static_cast<int>(write_split), at::cuda::getCurrentCUDAStream());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
@@ -1270,6 +1350,61 @@ void transpose_split(const torch::Tensor& ops, const torch::Tensor& tiles, int64
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
+// Each spec: (src [d, d], dst, dst_t | None, meta): see PairOp.  Returns (ops, bands, number of bands, tiles, number of tiles).
+std::tuple<torch::Tensor, torch::Tensor, int64_t, torch::Tensor, int64_t> build_pair_table(const std::vector<py::tuple>& specs) {
+  std::vector<PairOp> ops(specs.size());
+  std::vector<int2> bands;
+  std::vector<int4> tiles;
+  torch::Device device(torch::kCPU);
+  for (size_t i = 0; i < specs.size(); ++i) {
+    const py::tuple& s = specs[i];
+    TORCH_CHECK(s.size() == 4, "pair spec must have 4 fields");
+    const auto src = s[0].cast<torch::Tensor>();
+    TORCH_CHECK(src.is_cuda() && src.scalar_type() == torch::kFloat32 && src.dim() == 2 && src.stride(1) == 1 &&
+                    src.size(0) == src.size(1),
+                "pair source must be a square fp32 CUDA matrix");
+    device = src.device();
+    PairOp& op = ops[i];
+    op.src = src.data_ptr<float>();
+    op.d = static_cast<int>(src.size(0));
+    op.ld_src = static_cast<int>(src.stride(0));
+    auto take = [&](int k, int* ld) -> float* {
+      const auto t = s[k].cast<std::optional<torch::Tensor>>();
+      *ld = 0;
+      if (!t.has_value()) return nullptr;
+      TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->dim() == 2 && t->stride(1) == 1 && t->size(0) >= op.d &&
+                      t->size(1) == t->stride(0) && t->stride(0) % kBK == 0 && t->stride(0) >= op.d &&
+                      reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0,
+                  "pair destination must be padded to a multiple of ", kBK, " columns");
+      *ld = static_cast<int>(t->stride(0));
+      return t->data_ptr<float>();
+    };
+    op.dst = take(1, &op.ld_dst);
+    op.dst_t = take(2, &op.ld_t);
+    TORCH_CHECK(op.dst != nullptr && op.dst_t != op.src, "pair destinations");
+    TORCH_CHECK(op.dst != op.src || op.ld_dst == op.ld_src, "a conversion in place keeps the pitch");
+    op.meta = fptr(s[3].cast<std::optional<torch::Tensor>>());
+    TORCH_CHECK(op.meta != nullptr, "pair meta data missing");
+    for (int r = 0; r < (op.d + 7) / 8; ++r) bands.push_back(make_int2(static_cast<int>(i), r));
+    for (int r = 0; r < (op.d + 31) / 32; ++r)
+      for (int c = 0; c < (op.d + 31) / 32; ++c) tiles.push_back(make_int4(static_cast<int>(i), r, c, 0));
+  }
+  auto d_ops = upload_bytes(ops.data(), ops.size() * sizeof(PairOp), device);
+  auto d_bands = upload_bytes(bands.data(), bands.size() * sizeof(int2), device);
+  auto d_tiles = upload_bytes(tiles.data(), tiles.size() * sizeof(int4), device);
+  return {d_ops, d_bands, static_cast<int64_t>(bands.size()), d_tiles, static_cast<int64_t>(tiles.size())};
+}
+
+void pair_mirrors(const torch::Tensor& ops, const torch::Tensor& bands, int64_t num_bands, const torch::Tensor& tiles,
+                  int64_t num_tiles) {
+  LaunchScope scope("ob200::pair_mirrors");
+  c10::cuda::CUDAGuard guard(ops.device());
+  launch_pair_mirrors(reinterpret_cast<const PairOp*>(ops.data_ptr()), reinterpret_cast<const int2*>(bands.data_ptr()),
+                      static_cast<int>(num_bands), reinterpret_cast<const int4*>(tiles.data_ptr()),
+                      static_cast<int>(num_tiles), at::cuda::getCurrentCUDAStream());
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+}
+
 void peer_copy(const torch::Tensor& table, const torch::Tensor& chunks, int64_t num_chunks) {
   LaunchScope scope("ob200::peer_copy");
   if (num_chunks == 0) return;
@@ -1312,12 +1447,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("pack_upper", &pack_upper);
   m.def("build_transpose_table", &build_transpose_table);
   m.def("transpose_split", &transpose_split);
+  m.attr("HALF_PAIR") = static_cast<int>(kGemmHalfPair);
+  static_assert(static_cast<int>(kGemmHalfPair) == static_cast<int>(kFormPair), "one code names the operand format");
+  m.def("build_pair_table", &build_pair_table);
+  m.def("pair_mirrors", &pair_mirrors);
   m.def("jacobi_eigh_into", &jacobi_eigh_into);
   m.def("run_gemm_plan_push", &run_gemm_plan_push);
   m.attr("FLAG_PEER_PUSH") = kFlagPeerPush;
   m.def("gathered_apply_scaled", &gathered_apply_scaled);
   m.def("build_block_table", &build_block_table);
-  m.def("grad_prologue", &grad_prologue);
+  m.def("grad_prologue", &grad_prologue, py::arg("blocks"), py::arg("tiles"), py::arg("num_tiles"), py::arg("grad_ptrs"),
+        py::arg("l2_weight_decay"), py::arg("beta1"), py::arg("beta3"), py::arg("bias_correction1"), py::arg("graft_kind"),
+        py::arg("graft_beta2"), py::arg("graft_weight"), py::arg("graft_bc2"), py::arg("graft_eps"), py::arg("write_split"),
+        py::arg("status"), py::arg("num_grad_peers"), py::arg("grad_scale"), py::arg("filtered_plain") = false);
   m.def("direction_epilogue", &direction_epilogue);
   m.def("gathered_apply", &gathered_apply);
   m.def("peer_barrier", &peer_barrier);

@@ -1,5 +1,6 @@
 // Grouped per-block pointwise kernels; see block_kernels.cuh.
 #include "block_kernels.cuh"
+#include "half_pair.cuh"
 #include "ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -116,9 +117,90 @@ __device__ __forceinline__ void load_recv4(float (&out)[4], const void* base, lo
   }
 }
 
+// Filtered gradient: EMA with beta1; the applied estimate uses beta3 on the old EMA.
+__device__ __forceinline__ float filtered_gradient(float m_old, float m_new, float g, const PrologueArgs& a) {
+  const float f = (a.beta3 != a.beta1) ? lerpf(m_old, g, 1.f - a.beta3) : m_new;
+  return f / a.bias_correction1;
+}
+
+// Block-wide maxima of NV values, each added to dst[k] (non-negative floats order like their bits).
+template <int NV>
+__device__ __forceinline__ void atomic_max_block(float (&v)[NV], float* const (&dst)[NV], float (&red)[NV][8]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] = fmaxf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+    if (lane == 0) red[k][warp] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    float m = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, red[threadIdx.x][w]);
+    if (m > 0.f && dst[threadIdx.x] != nullptr) atomicMax(reinterpret_cast<int*>(dst[threadIdx.x]), __float_as_int(m));
+  }
+  __syncthreads();
+}
+
+// Largest |gradient| and |filtered gradient| of every block, for the scale of their fp16 pairs.  Reads what
+// the prologue reads again (at most 12 of its 12 + 20 bytes per element); up to the L2 capacity those
+// second reads do not reach HBM.  The pairs save 16 bytes per element in the prologue itself.  On one B200 the two
+// launches take 129 + 35 us for two GPT-2 layers (142 for the prologue that wrote tf32 pairs), which the
+// products more than give back.
+__global__ void __launch_bounds__(256) grad_amax_kernel(PrologueArgs a) {
+  __shared__ float red[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int t = blockIdx.x; t < a.num_tiles; t += gridDim.x) {
+    const TileRef ref = a.tiles[t];
+    const BlockDesc& b = a.blocks[ref.block];
+    if (b.aux == 1) continue;  // the block's other view of the same gradient
+    const float* src = a.grad_ptrs[b.grad_slot];
+    const int i0 = ref.ti * kTile, j = ref.tj * kWide + 4 * lane;
+    const int cnt = b.n - j < 4 ? b.n - j : 4;
+    const bool has_m1 = b.m1 != nullptr, l2 = a.l2_weight_decay != 0.f;
+    const bool vec = ((b.n | b.param_pitch | b.grad_offset) & 3) == 0 && aligned16(b.param) && aligned16(b.m1) && aligned16(src);
+    float g[4][4], mo[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + warp + 8 * r;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) g[r][k] = mo[r][k] = 0.f;
+      if (i >= b.m || cnt <= 0) continue;
+      const long long e = static_cast<long long>(i) * b.n + j;
+      const long long pe = static_cast<long long>(i) * b.param_pitch + j;
+      load4<false>(g[r], src + b.grad_offset + pe, vec, cnt);
+      if (l2) {
+        float w[4];
+        load4<false>(w, b.param + pe, vec, cnt);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) g[r][k] += a.l2_weight_decay * w[k];
+      }
+      if (has_m1) load4<false>(mo[r], b.m1 + e, vec, cnt);
+    }
+    float top[2] = {0.f, 0.f};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float gk = g[r][k];
+        const float f = has_m1 ? filtered_gradient(mo[r][k], lerpf(mo[r][k], gk, 1.f - a.beta1), gk, a) : gk;
+        top[0] = fmaxf(top[0], finite_abs(gk));
+        top[1] = fmaxf(top[1], finite_abs(f));
+      }
+    }
+    float* const dst[2] = {b.meta + kMetaGrad, b.meta + kMetaFiltered};
+    atomic_max_block<2>(top, dst, red);
+  }
+}
+
+// kPair: operands are written as scaled fp16 pairs, 4 bytes per element instead of the 8 of a tf32 pair.
+template <bool kPair>
 __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
-  __shared__ float t_hi[kTile][kWide + 1];
-  __shared__ float t_lo[kTile][kWide + 1];
+  // kPair: raw gradient, 16-byte column groups XOR-ed with the row's index / 4, which makes both the row-wise
+  // writes and the column-wise reads conflict-free.
+  __shared__ __align__(16) float t_hi[kTile][kPair ? kWide : kWide + 1];
+  __shared__ float t_lo[kPair ? 1 : kTile][kPair ? 1 : kWide + 1];
   __shared__ float red[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_src = a.num_grad_peers > 0 ? a.num_grad_peers : 1;
@@ -136,6 +218,8 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
     const bool l2 = a.l2_weight_decay != 0.f, graft = a.graft_kind != kGraftNone && b.norms != nullptr;
     bool vec = ((b.n | b.param_pitch | b.grad_offset) & 3) == 0 && aligned16(b.param) && aligned16(b.m1) && aligned16(b.v);
     for (int r = 0; r < n_src; ++r) vec = vec && aligned16(srcs[r]);
+    const float scale_g = kPair ? pair_scale(b.meta[kMetaGrad]) : 1.f;
+    const float scale_f = kPair ? pair_scale(b.meta[kMetaFiltered]) : 1.f;
 
     // ---- all loads of the tile first (4 rows x up to 4 arrays in flight per thread)
     float g[4][4], mo[4][4], vo[4][4];
@@ -186,22 +270,20 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
         const float gk = g[r][k];
         const bool live = on && k < cnt;
         bad |= live && !isfinite(gk);
-        if (a.write_split) {
+        if (!kPair && a.form == kFormSplit) {
           hi[k] = tf32_round(gk);
           lo[k] = gk - hi[k];
         } else {
           hi[k] = gk;
           lo[k] = 0.f;
         }
-        // Filtered gradient: EMA with beta1; the applied estimate uses beta3 on the old EMA.
         float f = gk;
         mn[k] = 0.f;
         if (has_m1) {
           mn[k] = lerpf(mo[r][k], gk, 1.f - a.beta1);
-          f = (a.beta3 != a.beta1) ? lerpf(mo[r][k], gk, 1.f - a.beta3) : mn[k];
-          f = f / a.bias_correction1;
+          f = filtered_gradient(mo[r][k], mn[k], gk, a);
         }
-        if (a.write_split) {
+        if (!kPair && a.form == kFormSplit) {
           fh[k] = tf32_round(f);
           fl[k] = f - fh[k];
         } else {
@@ -222,18 +304,25 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
         const long long e = static_cast<long long>(i) * b.n + j;
         if (identity_p) store4(b.p + e, mo[r], vec, cnt);
         const long long o = static_cast<long long>(i) * b.n_pad + j;  // n_pad % 4 == 0: always 16-byte stores
-        if (b.g_hi != nullptr) {
+        if (!kPair && b.g_hi != nullptr) {
           store4(b.g_hi + o, hi, true, 4);
-          if (a.write_split) store4(b.g_lo + o, lo, true, 4);
+          if (a.form == kFormSplit) store4(b.g_lo + o, lo, true, 4);
         }
-        if (b.f_hi != nullptr) {
+        if (b.f_hi != nullptr && (!kPair || a.filtered_plain)) {
           store4(b.f_hi + o, fh, true, 4);
-          if (a.write_split) store4(b.f_lo + o, fl, true, 4);
+          if (!kPair && a.form == kFormSplit) store4(b.f_lo + o, fl, true, 4);
         }
         if (has_m1) store4(b.m1 + e, mn, vec, cnt);
         if (has_v) store4(b.v + e, vn, vec, cnt);
       }
-      if (want_t) {
+      if (kPair && i < b.m && j < b.n_pad) {  // up to the end of the last chunk: its padding is written as zeros
+        const long long row = static_cast<long long>(i) * b.n_pad;
+        if (b.g_hi != nullptr) store_pair4(b.g_hi + row, j, hi, scale_g);
+        if (b.f_hi != nullptr && !a.filtered_plain) store_pair4(b.f_hi + row, j, fh, scale_f);
+      }
+      if (kPair && want_t) {
+        *reinterpret_cast<float4*>(&t_hi[li][4 * (lane ^ (li >> 2))]) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+      } else if (want_t) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           t_hi[li][4 * lane + k] = hi[k];
@@ -249,11 +338,18 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
       for (int r = 0; r < 4; ++r) {
         const int lj = (threadIdx.x >> 3) + 32 * r;
         const int jj = j0 + lj;
-        if (jj < b.n && i0 + ii < b.m) {
+        if constexpr (kPair) {
+          // The 32 source rows are one chunk of row jj (m_pad % 32 == 0), rows beyond m its zero padding.
+          if (jj < b.n) {
+            const int col = ((lj & ~3) ^ (4 * (threadIdx.x & 7))) + (lj & 3);
+            const float h[4] = {t_hi[ii][col], t_hi[ii + 1][col], t_hi[ii + 2][col], t_hi[ii + 3][col]};
+            store_pair4(b.gt_hi + static_cast<long long>(jj) * b.m_pad, i0 + ii, h, scale_g);
+          }
+        } else if (jj < b.n && i0 + ii < b.m) {
           const long long o = static_cast<long long>(jj) * b.m_pad + i0 + ii;  // m_pad % 4 == 0
           const float h[4] = {t_hi[ii][lj], t_hi[ii + 1][lj], t_hi[ii + 2][lj], t_hi[ii + 3][lj]};
           store4(b.gt_hi + o, h, true, 4);
-          if (a.write_split) {
+          if (a.form == kFormSplit) {
             const float l[4] = {t_lo[ii][lj], t_lo[ii + 1][lj], t_lo[ii + 2][lj], t_lo[ii + 3][lj]};
             store4(b.gt_lo + o, l, true, 4);
           }
@@ -452,28 +548,35 @@ __global__ void __launch_bounds__(256) gathered_apply_kernel(const BlockDesc* __
   }
 }
 
+// kMeasure: only the largest |S| of each block, into its PairMeta.
+template <bool kMeasure>
 __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restrict__ blocks,
                                                         const TileRef* __restrict__ tiles, int num_tiles, float bc2,
-                                                        float inv_root, float eps, int write_split) {
+                                                        float inv_root, float eps, int form) {
+  __shared__ float red[1][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
     const TileRef ref = tiles[t];
     const BlockDesc& b = blocks[ref.block];
-    const int i0 = ref.ti * kTile, j = ref.tj * kWide + 4 * lane;
-    const int cnt = b.n - j < 4 ? b.n - j : 4;
     // The auxiliary descriptor of an order-3 block (its second 2-D view) carries no state: ev and p
     // are null there.
-    if (cnt <= 0 || b.aux == 1 || b.ev == nullptr) continue;
+    if (b.aux == 1 || b.ev == nullptr) continue;
+    const int i0 = ref.ti * kTile, j = ref.tj * kWide + 4 * lane;
+    const int cnt = b.n - j < 4 ? b.n - j : 4;
     const bool vec = (b.n & 3) == 0 && aligned16(b.ev) && aligned16(b.p);
+    const float scale = !kMeasure && form == kFormPair ? pair_scale(b.meta[kMetaScaled]) : 1.f;
     float ev[4][4], p[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = i0 + warp + 8 * r;
-      if (i >= b.m) continue;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ev[r][k] = p[r][k] = 0.f;
+      if (i >= b.m || cnt <= 0) continue;
       const long long e = static_cast<long long>(i) * b.n + j;
       load4<false>(ev[r], b.ev + e, vec, cnt);
       load4<false>(p[r], b.p + e, vec, cnt);
     }
+    float top[1] = {0.f};
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = i0 + warp + 8 * r;
@@ -486,12 +589,23 @@ __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restr
         const float base = ev[r][k] / bc2;
         const float pw = inv_root == 0.5f ? sqrtf(base) : inv_root == 0.25f ? sqrtf(sqrtf(base)) : powf(base, inv_root);
         const float s = k < cnt ? p[r][k] / (pw + eps) : 0.f;
-        hi[k] = write_split ? tf32_round(s) : s;
+        top[0] = fmaxf(top[0], finite_abs(s));
+        hi[k] = form == kFormSplit ? tf32_round(s) : s;
         lo[k] = s - hi[k];
       }
-      const long long o = static_cast<long long>(i) * b.n_pad + j;  // n_pad % 4 == 0
-      store4(b.f_hi + o, hi, true, 4);
-      if (write_split) store4(b.f_lo + o, lo, true, 4);
+      if constexpr (!kMeasure) {
+        const long long row = static_cast<long long>(i) * b.n_pad;  // n_pad % 4 == 0
+        if (form == kFormPair) {
+          if (j < b.n_pad) store_pair4(b.f_hi + row, j, hi, scale);
+        } else if (cnt > 0) {
+          store4(b.f_hi + row + j, hi, true, 4);
+          if (form == kFormSplit) store4(b.f_lo + row + j, lo, true, 4);
+        }
+      }
+    }
+    if constexpr (kMeasure) {
+      float* const dst[1] = {b.meta + kMetaScaled};
+      atomic_max_block<1>(top, dst, red);
     }
   }
 }
@@ -567,7 +681,12 @@ int grid_for(int num_tiles) {
 
 void launch_grad_prologue(const PrologueArgs& args, cudaStream_t stream) {
   if (args.num_tiles <= 0) return;
-  grad_prologue_kernel<<<grid_for(args.num_tiles), 256, 0, stream>>>(args);
+  if (args.form == kFormPair) {
+    grad_amax_kernel<<<grid_for(args.num_tiles), 256, 0, stream>>>(args);
+    grad_prologue_kernel<true><<<grid_for(args.num_tiles), 256, 0, stream>>>(args);
+  } else {
+    grad_prologue_kernel<false><<<grid_for(args.num_tiles), 256, 0, stream>>>(args);
+  }
 }
 
 void launch_direction_epilogue(const EpilogueArgs& args, cudaStream_t stream) {
@@ -580,10 +699,13 @@ void launch_direction_epilogue(const EpilogueArgs& args, cudaStream_t stream) {
 }
 
 void launch_eig_scale(const BlockDesc* blocks, const TileRef* tiles, int num_tiles, float bias_correction2,
-                      float inv_root, float epsilon, int write_split, cudaStream_t stream) {
+                      float inv_root, float epsilon, int form, cudaStream_t stream) {
   if (num_tiles <= 0) return;
-  eig_scale_kernel<<<grid_for(num_tiles), 256, 0, stream>>>(blocks, tiles, num_tiles, bias_correction2, inv_root,
-                                                            epsilon, write_split);
+  const int grid = grid_for(num_tiles);
+  if (form == kFormPair) {
+    eig_scale_kernel<true><<<grid, 256, 0, stream>>>(blocks, tiles, num_tiles, bias_correction2, inv_root, epsilon, form);
+  }
+  eig_scale_kernel<false><<<grid, 256, 0, stream>>>(blocks, tiles, num_tiles, bias_correction2, inv_root, epsilon, form);
 }
 
 void launch_mode_switch(const BlockDesc* blocks, const TileRef* tiles, int num_tiles, float coeff, int send_dtype,

@@ -52,6 +52,17 @@ struct BlockDesc {
                           // 2: a block none of whose dims is preconditioned: the prologue writes the
                           // filtered gradient to p and its squared norm to norms[1] itself
   int pad_;
+  float* meta;            // half pairs: PairMeta of the gradient, the filtered gradient and the scaled
+                          // direction (kMeta*, two floats each), zeroed at the start of the step
+};
+
+constexpr int kMetaGrad = 0, kMetaFiltered = 2, kMetaScaled = 4;
+
+// Form of the operand arrays the pointwise kernels write.
+enum OperandForm : int {
+  kFormPlain = 0,  // raw fp32 in the *_hi arrays, no *_lo
+  kFormSplit = 1,  // tf32 (hi, lo) fp32 arrays
+  kFormPair = 2,   // scaled fp16 pairs in the *_hi arrays (half_pair.cuh), no *_lo; pitches are multiples of 32
 };
 
 struct TileRef {
@@ -77,7 +88,9 @@ struct PrologueArgs {
   float bias_correction1;         // 1 - beta3 * beta1^(t-1), or 1
   int graft_kind;
   float graft_beta2, graft_weight, graft_bias_correction2, graft_epsilon;
-  int write_split;                // 0: store raw fp32 into the *_hi arrays and skip *_lo (tf32 mode)
+  int form;                       // OperandForm
+  int filtered_plain;             // kFormPair: f_hi receives the raw filtered gradient (a step that only
+                                  // takes the grafting direction from it)
   int* status;                    // bit 1 set when a gradient holds NaN/Inf
 };
 
@@ -105,10 +118,11 @@ struct EpilogueArgs {
 };
 
 // eig_scale: S = P / ((ev / bc2)^(1/root) + eps) on the projected filtered gradient held in
-// BlockDesc::p, written as the (hi, lo) operand pair into f_hi / f_lo for the unprojection GEMMs
+// BlockDesc::p, written as the operand of the unprojection GEMMs into f_hi / f_lo; with half pairs a
+// first launch finds the largest |S| of each block, from which the pairs' scale follows
 // (reference: shampoo_preconditioner_list.py:1920-1942).
 void launch_eig_scale(const BlockDesc* blocks, const TileRef* tiles, int num_tiles, float bias_correction2,
-                      float inv_root, float epsilon, int write_split, cudaStream_t stream);
+                      float inv_root, float epsilon, int form, cudaStream_t stream);
 
 // mode_switch: W <- W + c (Z - W) for every block, the train()/eval() switch of the primal
 // averaging schemes; with BlockDesc::send the delta goes to the gather buffer instead
@@ -124,6 +138,7 @@ constexpr int kErrPeerTimeout = 4;  // a bounded wait on a peer's flag expired
 void launch_peer_barrier(int* local_flags, const unsigned long long* peer_flag_bases, int my_rank, int world,
                          int seq, int* status, cudaStream_t stream);
 
+// kFormPair: two launches, the first of which finds the largest gradient and filtered gradient of each block.
 void launch_grad_prologue(const PrologueArgs& args, cudaStream_t stream);
 void launch_direction_epilogue(const EpilogueArgs& args, cudaStream_t stream);
 

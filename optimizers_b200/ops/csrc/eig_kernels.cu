@@ -1,5 +1,6 @@
 // See eig_kernels.cuh.
 #include "eig_kernels.cuh"
+#include "half_pair.cuh"
 #include "ptx.cuh"
 
 namespace ob200 {
@@ -726,6 +727,62 @@ __global__ void __launch_bounds__(256) transpose_split_kernel(const TransposeOp*
   }
 }
 
+// A warp per row.  The row norm bounds the products' results more tightly than the largest entry does, and
+// with it the scale of a chained product's output.
+__global__ void __launch_bounds__(256) pair_measure_kernel(const PairOp* __restrict__ ops, const int2* __restrict__ bands,
+                                                           int num_bands) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int t = blockIdx.x; t < num_bands; t += gridDim.x) {
+    const int2 ref = bands[t];
+    const PairOp op = ops[ref.x];
+    const int row = ref.y * 8 + warp;
+    if (row >= op.d) continue;
+    const float* src = op.src + static_cast<long long>(row) * op.ld_src;
+    float top = 0.f, sq = 0.f;
+    for (int j = lane; j < op.d; j += 32) {
+      const float x = finite_abs(src[j]);
+      top = fmaxf(top, x);
+      sq = fmaf(x, x, sq);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    }
+    if (lane == 0 && top > 0.f) {
+      atomicMax(reinterpret_cast<int*>(op.meta), __float_as_int(top));
+      atomicMax(reinterpret_cast<int*>(op.meta + 1), __float_as_int(sq));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) pair_convert_kernel(const PairOp* __restrict__ ops, const int4* __restrict__ tiles,
+                                                           int num_tiles) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;     // 32 x 8: loads
+  const int row = threadIdx.x >> 3, g = 4 * (threadIdx.x & 7);  // four consecutive columns: stores
+  for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+    const int4 ref = tiles[t];
+    const PairOp op = ops[ref.x];
+    const int r0 = ref.y * 32, c0 = ref.z * 32;
+    for (int k = ty; k < 32; k += 8) {
+      const int r = r0 + k, c = c0 + tx;
+      tile[k][tx] = (r < op.d && c < op.d) ? op.src[static_cast<long long>(r) * op.ld_src + c] : 0.f;
+    }
+    __syncthreads();
+    const float s = pair_scale(op.meta[0]);
+    if (r0 + row < op.d) {
+      const float v[4] = {tile[row][g], tile[row][g + 1], tile[row][g + 2], tile[row][g + 3]};
+      store_pair4(op.dst + static_cast<long long>(r0 + row) * op.ld_dst, c0 + g, v, s);
+    }
+    if (op.dst_t != nullptr && c0 + row < op.d) {
+      const float v[4] = {tile[g][row], tile[g + 1][row], tile[g + 2][row], tile[g + 3][row]};
+      store_pair4(op.dst_t + static_cast<long long>(c0 + row) * op.ld_t, r0 + g, v, s);
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace
 
 void launch_householder_panel(const QrPanelDesc* descs, int count, cudaStream_t stream) {
@@ -795,6 +852,14 @@ void launch_transpose_split(const TransposeOp* ops, const int4* tiles, int num_t
   if (num_tiles <= 0) return;
   const int cap = sm_count() * 16;
   transpose_split_kernel<<<num_tiles < cap ? num_tiles : cap, 256, 0, stream>>>(ops, tiles, num_tiles);
+}
+
+void launch_pair_mirrors(const PairOp* ops, const int2* bands, int num_bands, const int4* tiles, int num_tiles,
+                         cudaStream_t stream) {
+  if (num_tiles <= 0) return;
+  const int cap = sm_count() * 8;
+  pair_measure_kernel<<<num_bands < cap ? num_bands : cap, 256, 0, stream>>>(ops, bands, num_bands);
+  pair_convert_kernel<<<num_tiles < 2 * cap ? num_tiles : 2 * cap, 256, 0, stream>>>(ops, tiles, num_tiles);
 }
 
 }  // namespace ob200

@@ -132,4 +132,18 @@ struct TransposeOp {
 };
 void launch_transpose_split(const TransposeOp* ops, const int4* tiles, int num_tiles, cudaStream_t stream);
 
+// Operand mirrors as scaled fp16 pairs (half_pair.cuh): dst = the d x d matrix at src (dst may be src: each
+// 32 x 32 tile is replaced by its own chunks), dst_t (may be null) its transpose.  A first launch over
+// 8-row bands finds the largest entry and the largest row norm and puts them into `meta`, which the
+// caller has zeroed.
+struct PairOp {
+  const float* src;
+  float* dst;
+  float* dst_t;
+  float* meta;
+  int d, ld_src, ld_dst, ld_t;
+};
+void launch_pair_mirrors(const PairOp* ops, const int2* bands, int num_bands, const int4* tiles, int num_tiles,
+                         cudaStream_t stream);
+
 }  // namespace ob200

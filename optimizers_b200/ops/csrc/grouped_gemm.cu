@@ -4,6 +4,7 @@
 // shampoo_preconditioner_list.py:1499-1507 factor Gram matrices, :1563-1578 preconditioner
 // application) together with the packing / EMA / norm kernels around them (:1525-1539).
 #include "grouped_gemm.cuh"
+#include "half_pair.cuh"
 #include "ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -18,13 +19,18 @@ constexpr int kEpilogueWarps = 4;
 constexpr int kTileBytesA = kBM * kBK * 4;  // 16 KiB
 constexpr int kTileBytesB = kBN * kBK * 4;  // 16 KiB
 constexpr int kStagePitch = 33;             // floats per staged row: conflict-free transposition
-constexpr int kAccumCols = 2 * kBN;         // two accumulator buffers
 constexpr uint32_t kIdesc = make_idesc(/*tf32*/ 2, kBM, kBN);
+constexpr uint32_t kIdescHalf = make_idesc(/*f16*/ 0, kBM, kBN);
+constexpr uint32_t kIdescHalfWide = make_idesc(/*f16*/ 0, kBM, 2 * kBN);
 
-template <int kSplit>
+template <int kMode>
 struct Cfg {
-  static constexpr int kStageBytes = (kTileBytesA + kTileBytesB) * (kSplit ? 2 : 1);
-  static constexpr int kStages = kSplit ? 3 : 6;
+  static constexpr int kAccCols = kMode == kGemmHalfPair ? 2 * kBN : kBN;  // columns of one accumulator buffer
+  static constexpr int kTmemCols = 2 * kAccCols;                           // two accumulator buffers
+  // tf32x3: hi and lo of both operands; half pairs: one A tile and up to two B tiles (256 columns)
+  static constexpr int kStageBytes =
+      kMode == kGemmTf32x3 ? 2 * (kTileBytesA + kTileBytesB) : kTileBytesA + (kMode == kGemmHalfPair ? 2 : 1) * kTileBytesB;
+  static constexpr int kStages = kMode == kGemmTf32x3 ? 3 : kMode == kGemmHalfPair ? 4 : 6;
   static constexpr int kStagingBytes = kEpilogueWarps * 32 * kStagePitch * 4;
   static constexpr int kBarrierBytes = 256;
   // 1024 B of slack so the stage buffers can be aligned for the 128-byte swizzle.
@@ -33,12 +39,13 @@ struct Cfg {
 
 // kPush: instantiation whose epilogue also stores into the peers' gather buffers; kept apart so
 // that the store loop of the common instantiation is not burdened with it.
-template <int kSplit, bool kPush>
+template <int kMode, bool kPush>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __restrict__ tiles, int num_tiles,
                     float alpha, float beta, float gamma, int* __restrict__ status, const PeerPush push) {
-  using C = Cfg<kSplit>;
+  using C = Cfg<kMode>;
   constexpr int kStages = C::kStages;
+  constexpr bool kSplit = kMode == kGemmTf32x3, kHalf = kMode == kGemmHalfPair;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -69,7 +76,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
     fence_proxy_async_smem();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_holder, kAccumCols);
+    tmem_alloc(tmem_holder, C::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -93,11 +100,13 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
             break;
           }
           uint8_t* s = stage_base + stage * C::kStageBytes;
-          mbar_arrive_expect_tx(&full_bar[stage], C::kStageBytes);
+          const bool wide = kHalf && tile.cols > kBN;
+          mbar_arrive_expect_tx(&full_bar[stage], kHalf && !wide ? kTileBytesA + kTileBytesB : C::kStageBytes);
           const int ak = p->a_k0 + kb * kBK, bk = p->b_k0 + kb * kBK;
           const int ar = p->a_row0 + tile.m0, br = p->b_row0 + tile.n0;
           tma_load_2d(s, p->a_hi, &full_bar[stage], ak, ar);
           tma_load_2d(s + kTileBytesA, p->b_hi, &full_bar[stage], bk, br);
+          if (wide) tma_load_2d(s + kTileBytesA + kTileBytesB, p->b_hi, &full_bar[stage], bk, br + kBN);
           if (kSplit) {
             tma_load_2d(s + kTileBytesA + kTileBytesB, p->a_lo, &full_bar[stage], ak, ar);
             tma_load_2d(s + 2 * kTileBytesA + kTileBytesB, p->b_lo, &full_bar[stage], bk, br);
@@ -122,7 +131,8 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
         const int buf = it & 1;
         if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + buf * kBN;
+        const uint32_t d_tmem = tmem_base + buf * C::kAccCols;
+        const uint32_t idesc_half = tile.cols > kBN ? kIdescHalfWide : kIdescHalf;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
             ok = false;
@@ -132,6 +142,23 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           const uint32_t s = smem_u32(stage_base + stage * C::kStageBytes);
           const uint64_t a_hi = make_kmajor_sw128_desc(s);
           const uint64_t b_hi = make_kmajor_sw128_desc(s + kTileBytesA);
+          if constexpr (kHalf) {
+            // A row is [32 fp16 hi | 32 fp16 lo]: K steps of 16 at byte offsets 0 and 32, the lo
+            // halves 64 bytes further.
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const uint64_t hi = static_cast<uint64_t>(k * 2), lo = static_cast<uint64_t>(4 + k * 2);
+              umma_f16(d_tmem, a_hi + lo, b_hi + hi, idesc_half, (kb | k) != 0);
+              umma_f16(d_tmem, a_hi + hi, b_hi + hi, idesc_half, 1);
+              umma_f16(d_tmem, a_hi + hi, b_hi + lo, idesc_half, 1);
+            }
+            umma_commit(&empty_bar[stage]);
+            if (++stage == kStages) {
+              stage = 0;
+              phase ^= 1;
+            }
+            continue;
+          }
           const uint64_t a_lo = make_kmajor_sw128_desc(s + kTileBytesA + kTileBytesB);
           const uint64_t b_lo = make_kmajor_sw128_desc(s + 2 * kTileBytesA + kTileBytesB);
 #pragma unroll
@@ -177,6 +204,22 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       tc_fence_after_sync();
       const int row0 = tile.m0 + q * 32;
       float sq = 0.f, tr = 0.f;
+      // Half pairs: the accumulator holds (s_a a)(s_b b); the powers of two are taken out one after the
+      // other, since their product may leave the range of fp32.  The scale of a split output follows
+      // from |c_ij| <= ||a_i|| ||b_j||, the same for every tile, so whoever is here writes it.
+      float inv_a = 1.f, inv_b = 1.f, scale_d = 1.f;
+      if constexpr (kHalf) {
+        inv_a = pair_inverse_scale(p->a_meta[0]);
+        inv_b = pair_inverse_scale(p->b_meta[0]);
+        if (flags & kFlagSplitOut) {
+          const float bound = fabsf(alpha) * pair_row_bound(p->a_meta, p->K) * pair_row_bound(p->b_meta, p->K);
+          scale_d = pair_scale(bound);
+          if (threadIdx.x == 64) {
+            p->d_meta[0] = bound;
+            p->d_meta[1] = 0.f;
+          }
+        }
+      }
       // Symmetric result (kFlagMirror): only entries on or above the diagonal are taken from the
       // accumulator; every 32 x 32 chunk strictly above the diagonal is also stored transposed and
       // the chunks on the diagonal are symmetrised, so the stored matrix is symmetric bit for bit
@@ -186,7 +229,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       const bool diag_tile = sym && tile.n0 == tile.m0;
       if (row0 < M) {
 #pragma unroll 1
-        for (int c = 0; c < kBN / 32; ++c) {
+        for (int c = 0; c < (kHalf ? tile.cols / 32 : kBN / 32); ++c) {
           const int col0 = tile.n0 + c * 32;
           if (col0 >= N) break;
           if ((flags & kFlagPackedC) && col0 + 31 < row0) continue;  // chunk strictly below the diagonal
@@ -194,8 +237,22 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           const bool mirror = sym && (!diag_tile || c > q);
           const bool diag_chunk = diag_tile && c == q;
           float v[32];
-          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * kBN + c * 32, v);
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
           float sq_chunk = 0.f;
+          if constexpr (kHalf) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = (v[j] * inv_a) * inv_b;
+            if (flags & kFlagSplitOut) {
+              // One thread owns the 128-byte chunk of its row: 32 hi, then 32 lo (zero beyond N, which
+              // the next product reads as K padding).
+              if (row0 + lane < M) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = col0 + j < N ? alpha * v[j] : 0.f;
+                store_pair_chunk(Dhi + static_cast<long long>(row0 + lane) * ldd + col0, v, scale_d);
+              }
+              continue;
+            }
+          }
           // Fast path: the thread that holds row (row0 + lane) of the accumulator stores its 32
           // consecutive columns itself with 16-byte accesses (C, then the (hi, lo) pair), and
           // stores the transposed copy of a symmetric result one column at a time, where the 32
@@ -420,38 +477,39 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
   }
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, kAccumCols);
+    tmem_dealloc(tmem_base, C::kTmemCols);
   }
 }
 
-template <int kSplit, bool kPush>
+template <int kMode, bool kPush>
 void launch_impl(const GemmProblem* problems, const GemmTile* tiles, int num_tiles, float alpha, float beta,
                  float gamma, int* status, int max_ctas, cudaStream_t stream, const PeerPush& push) {
-  using C = Cfg<kSplit>;
+  using C = Cfg<kMode>;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(grouped_gemm_kernel<kSplit, kPush>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kPush>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     configured = true;
   }
   const int grid = num_tiles < max_ctas ? num_tiles : max_ctas;
-  grouped_gemm_kernel<kSplit, kPush><<<grid, kThreads, C::kSmemBytes, stream>>>(problems, tiles, num_tiles, alpha,
+  grouped_gemm_kernel<kMode, kPush><<<grid, kThreads, C::kSmemBytes, stream>>>(problems, tiles, num_tiles, alpha,
                                                                                beta, gamma, status, push);
 }
 
 }  // namespace
 
 void launch_grouped_gemm(const GemmProblem* problems, const GemmTile* tiles, int num_tiles, float alpha, float beta,
-                         bool split, int* status, int max_ctas, cudaStream_t stream, const PeerPush* push, float gamma) {
+                         GemmMode mode, int* status, int max_ctas, cudaStream_t stream, const PeerPush* push, float gamma) {
   if (num_tiles <= 0) return;
   PeerPush none{};
   const PeerPush& pp = push != nullptr ? *push : none;
   const bool pushing = pp.num_peers > 0;
-  if (split) {
-    if (pushing) launch_impl<1, true>(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp);
-    else launch_impl<1, false>(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp);
+  auto go = [&](auto launch) { launch(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp); };
+  if (mode == kGemmHalfPair) {
+    pushing ? go(launch_impl<kGemmHalfPair, true>) : go(launch_impl<kGemmHalfPair, false>);
+  } else if (mode == kGemmTf32x3) {
+    pushing ? go(launch_impl<kGemmTf32x3, true>) : go(launch_impl<kGemmTf32x3, false>);
   } else {
-    if (pushing) launch_impl<0, true>(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp);
-    else launch_impl<0, false>(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp);
+    pushing ? go(launch_impl<kGemmTf32, true>) : go(launch_impl<kGemmTf32, false>);
   }
 }
 

@@ -1,15 +1,24 @@
 // Grouped "TN" GEMM on the 5th-generation tensor cores:  C_g = beta * C_g + alpha * A_g * B_g^T
-// for a table of independent problems, where A_g is [M,K] and B_g is [N,K], both K-major fp32.
+// for a table of independent problems, where A_g is [M,K] and B_g is [N,K], both K-major.
 //
-// Two accuracy modes.  kSplit == 1: each operand arrives as a (hi, lo) pair with
-// hi = tf32_round(x), lo = x - hi, and every K step issues three tf32 products
+// Operand formats (GemmMode).  kGemmTf32x3: each operand arrives as a (hi, lo) pair of fp32 arrays
+// with hi = tf32_round(x), lo = x - hi, and every K step issues three tf32 products
 // (hi*hi + hi*lo + lo*hi) into the same fp32 TMEM accumulator, which restores fp32-grade
-// accuracy.  kSplit == 0: one tf32 product on the raw fp32 operands.
+// accuracy.  kGemmTf32: one tf32 product on the raw fp32 operands.  kGemmHalfPair: the same three
+// products at the fp16 rate, twice that of tf32, on interleaved scaled fp16 pairs (half_pair.cuh):
+// hi and lo of 32 consecutive K elements share one 128-byte swizzle row, so an operand is one array of
+// 4 bytes per element, half of the tf32 pair's.  Both splits carry 11 + 11 significant bits; the
+// fp16 one rounds lo where the tensor core truncates a tf32 lo, and sums 16 products instead of 8
+// before each (truncating) accumulation, so its error is the smaller one.  Measured on one B200 (the three
+// products counted): 16 products of 2048^3 in 581 us instead of 1128 (1420 TFLOP/s against 730; cuBLAS bf16
+// reaches 1590), 6 of 768^3 in 27 us instead of 42, relative error against fp64 at K = 2048 7.2e-6 instead
+// of 1.4e-5.
 //
 // Structure (one persistent CTA per SM, 192 threads):
-//   warp 0      TMA producer: cp.async.bulk.tensor tiles of 128 x 32 fp32 with 128-byte swizzle
-//   warp 1      MMA issuer: tcgen05.mma 128x128x8 kind::tf32, accumulators in TMEM, two
-//               accumulator buffers so the epilogue of one tile overlaps the next tile's MMAs
+//   warp 0      TMA producer: cp.async.bulk.tensor tiles of 128 rows x 128 bytes, 128-byte swizzle
+//   warp 1      MMA issuer: tcgen05.mma 128x128x8 kind::tf32, or 128x128x16 / 128x256x16 kind::f16,
+//               accumulators in TMEM, two accumulator buffers so the epilogue of one tile overlaps
+//               the next tile's MMAs
 //   warps 2..5  epilogue: tcgen05.ld, transpose through shared memory, then coalesced global
 //               access with the fused options below.
 //
@@ -73,7 +82,10 @@ struct alignas(128) GemmProblem {
   int ldc;  // row pitch of C in elements (full mode); N in packed mode
   int ldd;  // row pitch of d_hi / d_lo
   int flags;
-  int pad_[2];
+  // kGemmHalfPair: PairMeta of the operands (read) and of the split output (written, kFlagSplitOut)
+  const float* a_meta;
+  const float* b_meta;
+  float* d_meta;
   long long push_offset;  // byte offset of the problem's slot inside the gather buffers (kFlagPeerPush)
 };
 
@@ -89,16 +101,18 @@ struct GemmTile {
   int problem;
   int m0;  // first row of the tile
   int n0;  // first column of the tile
-  int pad_;
+  int cols;  // 128, or 256 (kGemmHalfPair only)
 };
+
+enum GemmMode : int { kGemmTf32 = 0, kGemmTf32x3 = 1, kGemmHalfPair = 2 };
 
 constexpr int kBM = 128;
 constexpr int kBN = 128;
-constexpr int kBK = 32;  // fp32 elements = 128 bytes = one swizzle row
+constexpr int kBK = 32;  // fp32 elements (or fp16 pairs) = 128 bytes = one swizzle row
 
 // Host-side launch.  `status` is a device int the kernel writes a non-zero error code to.
 void launch_grouped_gemm(const GemmProblem* problems, const GemmTile* tiles, int num_tiles, float alpha, float beta,
-                         bool split, int* status, int max_ctas, cudaStream_t stream, const PeerPush* push = nullptr,
+                         GemmMode mode, int* status, int max_ctas, cudaStream_t stream, const PeerPush* push = nullptr,
                          float gamma = 0.f);
 
 }  // namespace ob200
