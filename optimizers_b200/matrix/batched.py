@@ -25,6 +25,7 @@ block's tolerated consecutive failures.
 from __future__ import annotations
 
 import logging
+import math
 import threading
 from concurrent.futures import ThreadPoolExecutor
 from types import SimpleNamespace
@@ -667,41 +668,49 @@ def batched_newton_refresh(
         it.converged, it.last_err, it.iters = False, float("inf"), 0
         it.Ar = None
         items.append(it)
-    finite = _all_finite([it.A for it in items])
-    for it, ok in zip(items, finite):
-        if not ok:
+    # One read for all factors: largest entries (finite?) and, for Newton, the norms of the ridged factors.
+    mats = [it.A for it in items]
+    measures = torch._foreach_norm(mats, float("inf"))
+    if higher is None:
+        torch._foreach_add_([A.diagonal() for A in mats], [float(it.block.factors.epsilon) for it in items])
+        measures += torch._foreach_norm(mats)
+    measures = torch.stack(measures).cpu().tolist()
+    for it, top in zip(items, measures):
+        if not math.isfinite(top):
             index = it.block.factors.factor_matrix_indices[it.k]
             raise PreconditionerValueError(f"Encountered nan/inf values in factor matrix {index}!")
 
-    # Initial iterates: z = (p+1) / (2 ||A||_F), X = z^(1/p) I, M = z A  (no host synchronisation).
+    # Initial iterates: z = (p+1) / (2 ||A||_F), X = z^(1/p) I, M = z A.  The iteration's matrices come from one
+    # allocation and the iterates of all factors from one launch: a dozen tensors per factor, each with a fill
+    # launch of its own, were half of a refresh's host time.
     errs = torch.zeros(len(items), device=device)
+    sizes = [it.d for it in items for _ in range(5)]
+    pairs = [(hi, lo) for _, hi, lo in ext.alloc_mat_batch(sizes, sizes, False, True, device)]
+    start = []
     for n, it in enumerate(items):
+        it.X, it.M, it.Mp = pairs[5 * n : 5 * n + 2], pairs[5 * n + 2 : 5 * n + 4], pairs[5 * n + 4]
+        it.pw = {}
+        it.err = errs[n : n + 1]
+        if higher is None:
+            norm = measures[len(items) + n]
+            z = (it.root + 1) / (2 * norm) if norm > 0.0 else float("inf")
+            start.append((it.A, *it.X[0], None, 0.0, z ** (1.0 / it.root)))
+            start.append((it.A, *it.M[0], None, z, 0.0))
+            continue
         d, p = it.d, it.root
         A_r = it.A.clone()
-        if higher is None:
-            A_r.diagonal().add_(it.block.factors.epsilon)
-            z = (p + 1) / (2 * torch.linalg.norm(A_r))
-        else:
-            lam = torch.linalg.matrix_norm(it.A, torch.inf)
-            A_r.diagonal().add_(torch.clamp(lam * higher.rel_epsilon, min=higher.abs_epsilon))
-            z = torch.reciprocal(torch.trace(A_r))
-            it.Ar = _pair(d, device, split)  # the verification at the end multiplies X^p by it
-            ext.tf32_split(A_r, *_v(it.Ar, d))
-        it.X = [_pair(d, device, split), _pair(d, device, split)]
-        it.M = [_pair(d, device, split), _pair(d, device, split)]
-        it.Mp = _pair(d, device, split)
-        it.pw = {}
+        lam = torch.linalg.matrix_norm(it.A, torch.inf)
+        A_r.diagonal().add_(torch.clamp(lam * higher.rel_epsilon, min=higher.abs_epsilon))
+        z = torch.reciprocal(torch.trace(A_r))
+        it.Ar = _pair(d, device, split)  # the verification at the end multiplies X^p by it
+        ext.tf32_split(A_r, *_v(it.Ar, d))
         x0 = torch.zeros(d, d, device=device)
         x0.diagonal().fill_(1.0)
         x0 *= z ** (1.0 / p)
-        m0 = A_r * z
-        for src, dst in ((x0, it.X[0]), (m0, it.M[0])):
-            hi, lo = _v(dst, d)
-            if split:
-                ext.tf32_split(src, hi, lo)
-            else:
-                hi.copy_(src)
-        it.err = errs[n : n + 1]
+        ext.tf32_split(x0, *it.X[0])
+        ext.tf32_split(A_r * z, *it.M[0])
+    if start:
+        ext.shift_scale_split(*ext.build_sym_table(start))
     order = higher.order if higher is not None else 0
     return _newton_iterate(ext, items, errs, split, status, max_iterations, tolerance, check_every, blocks, order)
 
@@ -728,16 +737,21 @@ def _newton_iterate(ext, items, errs, split, status, max_iterations, tolerance, 
 
     # results -> packed checkpoint state; one finiteness read
     good = [it for it in items if id(it) not in failures]
-    flags = []
-    for it in good:
-        kf = it.block.factors
-        hi, lo = _v(it.X, it.d)
-        full = hi + lo if lo is not None else hi
-        state = kf.inv_factor_matrices[it.k]
-        state.copy_(kf.pack(full).to(dtype=state.dtype))
-        flags.append(torch.isfinite(state).all())
-    if flags:
-        for it, ok in zip(good, torch.stack(flags).cpu().tolist()):
+    if good:
+        pairs = [_v(it.X, it.d) for it in good]
+        full = torch._foreach_add([hi for hi, _ in pairs], [lo for _, lo in pairs])
+        states, pack_specs = [], []
+        for it, X in zip(good, full, strict=True):
+            kf = it.block.factors
+            state = kf.inv_factor_matrices[it.k]
+            states.append(state)
+            if state.is_cuda and state.dtype == torch.float32 and (state.dim() == 1 or state.stride(-1) == 1) and X.stride(-1) == 1:
+                pack_specs.append((X, state))
+            else:
+                state.copy_(kf.pack(X).to(dtype=state.dtype))
+        if pack_specs:
+            ext.pack_upper(*ext.build_pack_table(pack_specs))
+        for it, ok in zip(good, _all_finite(states)):
             if not ok:
                 index = it.block.factors.factor_matrix_indices[it.k]
                 raise PreconditionerValueError(f"Encountered nan or inf values in matrices of factor matrix {index}!")
@@ -763,16 +777,17 @@ def _newton_run_chunk(ext, chunk, p, errs, split, status, max_iterations, tolera
     horner = max(order - 2, 0)  # products per higher-order step that build M_p
     if order:
         check_every = 1  # the stopping rule compares consecutive errors
-    for it in chunk:
-        d = it.d
-        it.pw = {e: _pair(d, device, split) for e, _, _ in chain}
-        # full-precision copies of M (source of the affine step and of the error measure)
-        it.A = [torch.zeros(d, _pad4(d), device=device), torch.zeros(d, _pad4(d), device=device)]
-        hi, lo = _v(it.M[0], d)
-        it.A[0][:, :d].copy_(hi + lo if lo is not None else hi)
+    sizes = [it.d for it in chunk]
+    # full-precision copies of M (source of the affine step and of the error measure)
+    copies = [[full for full, _, _ in ext.alloc_mat_batch(sizes, sizes, True, False, device)] for _ in range(2)]
+    scratch = [[(hi, lo) for _, hi, lo in ext.alloc_mat_batch(sizes, sizes, False, True, device)] for _ in range(len(chain) + (3 if horner else 0))]
+    for n, it in enumerate(chunk):
+        it.A = [copies[0][n], copies[1][n]]
+        own = [batch[n] for batch in scratch]
+        it.pw = {e: own[i] for i, (e, _, _) in enumerate(chain)}
         if horner:
-            it.R = _pair(d, device, split)
-            it.T = [_pair(d, device, split) for _ in range(min(horner, 2))]
+            it.R, *it.T = own[len(chain) :]
+    torch._foreach_copy_(copies[0], torch._foreach_add([it.M[0][0] for it in chunk], [it.M[0][1] for it in chunk]))
 
     def gemm(a, b, out, d, c_full=None, flags=0):
         # Every product here is a polynomial in one symmetric matrix, hence symmetric: only the
