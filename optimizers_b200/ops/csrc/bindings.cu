@@ -293,7 +293,7 @@ class PlanBuilder {
           for (int step = 0; (upper ? band : 0) + step < p.N; step += widest) {
             for (int m0 = band; m0 < band_end; m0 += kBM) {
               const int n0 = (upper ? m0 : 0) + step;
-              if (n0 < p.N) tiles_.push_back({o.problem, m0, n0, p.N - n0 > kBN ? widest : kBN});
+              if (n0 < p.N) push_tile(o.problem, m0, n0, p.N - n0 > kBN ? widest : kBN);
             }
           }
         }
@@ -304,11 +304,12 @@ class PlanBuilder {
         for (int n0 = upper ? band : 0; n0 < p.N; n0 += kBN) {
           for (int m0 = band; m0 < band_end; m0 += kBM) {
             if (upper && n0 < m0) continue;
-            tiles_.push_back({o.problem, m0, n0, kBN});
+            push_tile(o.problem, m0, n0, kBN);
           }
         }
       }
     }
+    if (half_) split_along_k(first);
     launch_begin_ = static_cast<int>(problems_.size());
     return {first, static_cast<int64_t>(tiles_.size()) - first};
   }
@@ -320,7 +321,11 @@ class PlanBuilder {
     TORCH_CHECK(!problems_.empty(), "empty GEMM plan");
     const size_t table_bytes = problems_.size() * sizeof(GemmProblem);
     const size_t map_bytes = maps_.size() * sizeof(CUtensorMap);
-    auto buffer = torch::empty({static_cast<int64_t>(table_bytes + map_bytes)}, torch::dtype(torch::kUInt8).device(device_));
+    // [problems][tensor maps][counters of the split tiles: zero][their partial sums]
+    const size_t counter_bytes = (static_cast<size_t>(split_tiles_) * (kBM / 32) * sizeof(int) + 255) / 256 * 256;
+    const size_t host_bytes = table_bytes + map_bytes + counter_bytes;
+    auto buffer = torch::empty({static_cast<int64_t>(host_bytes + partial_floats_ * sizeof(float))},
+                               torch::dtype(torch::kUInt8).device(device_));
     const auto base = reinterpret_cast<uintptr_t>(buffer.data_ptr());
     TORCH_CHECK(base % 128 == 0, "problem table must be 128-byte aligned");
     const auto* dev_maps = reinterpret_cast<const CUtensorMap*>(base + table_bytes);
@@ -332,16 +337,72 @@ class PlanBuilder {
       p.b_hi = dev_maps + ix[2];
       p.b_lo = dev_maps + (ix[3] >= 0 ? ix[3] : ix[2]);
     }
-    auto host = torch::empty({static_cast<int64_t>(table_bytes + map_bytes)}, torch::dtype(torch::kUInt8).pinned_memory(true));
+    auto host = torch::empty({static_cast<int64_t>(host_bytes)}, torch::dtype(torch::kUInt8).pinned_memory(true));
     std::memcpy(host.data_ptr(), problems_.data(), table_bytes);
     std::memcpy(static_cast<uint8_t*>(host.data_ptr()) + table_bytes, maps_.data(), map_bytes);
-    buffer.copy_(host, /*non_blocking=*/true);
+    std::memset(static_cast<uint8_t*>(host.data_ptr()) + table_bytes + map_bytes, 0, counter_bytes);
+    buffer.narrow(0, 0, static_cast<int64_t>(host_bytes)).copy_(host, /*non_blocking=*/true);
+    for (GemmTile& t : tiles_) {
+      if (t.parts == 1) continue;
+      // until here the pointers hold the offsets split_along_k gave out
+      t.partial = reinterpret_cast<float*>(base + host_bytes) + reinterpret_cast<uintptr_t>(t.partial);
+      t.counter = reinterpret_cast<int*>(base + table_bytes + map_bytes) + reinterpret_cast<uintptr_t>(t.counter);
+    }
     auto d_tiles = upload_bytes(tiles_.data(), tiles_.size() * sizeof(GemmTile), device_);
     // The element type of the tile list tells a half-pair plan from an fp32 one (gemm_mode below).
     return {buffer, half_ ? d_tiles.view(torch::kInt32) : d_tiles};
   }
 
  private:
+  void push_tile(int problem, int m0, int n0, int cols) {
+    GemmTile t{};
+    t.problem = problem;
+    t.m0 = m0;
+    t.n0 = n0;
+    t.cols = cols;
+    t.kb1 = (problems_[problem].K + kBK - 1) / kBK;
+    t.parts = 1;
+    tiles_.push_back(t);
+  }
+
+  // Where a launch has too few tiles for the SMs, or single tiles with a K loop far longer than the others', the long
+  // loops are cut into parts of about an SM's share of all K blocks, of at least kMinPart blocks (a part
+  // costs a round trip of its accumulator through the L2, a few microseconds, as much as about 8 blocks) and
+  // at most kMaxParts (the last to arrive reads them all).  On one B200 the four launches of a step over ResNet
+  // weights, among them the Gram of a 3 x 98304 unfolding, went from 387 to 77 us.
+  void split_along_k(int64_t first) {
+    constexpr int kMinPart = 12, kMaxParts = 32;
+    const int sms = at::cuda::getDeviceProperties(device_.index())->multiProcessorCount;
+    int64_t total = 0;
+    for (size_t i = first; i < tiles_.size(); ++i) total += tiles_[i].kb1;
+    const int share = static_cast<int>(std::max<int64_t>(kMinPart, (total + sms - 1) / sms));
+    std::vector<GemmTile> out;
+    bool any = false;
+    for (size_t i = first; i < tiles_.size(); ++i) {
+      const GemmTile t = tiles_[i];
+      const int parts = 2 * t.kb1 > 3 * share ? std::min(kMaxParts, (t.kb1 + share - 1) / share) : 1;
+      for (int part = 0; part < parts; ++part) {
+        GemmTile u = t;
+        u.kb0 = static_cast<int>(static_cast<int64_t>(t.kb1) * part / parts);
+        u.kb1 = static_cast<int>(static_cast<int64_t>(t.kb1) * (part + 1) / parts);
+        u.part = part;
+        u.parts = parts;
+        u.partial = reinterpret_cast<float*>(static_cast<uintptr_t>(partial_floats_));  // offsets: see finalize
+        u.counter = reinterpret_cast<int*>(static_cast<uintptr_t>(split_tiles_ * (kBM / 32)));
+        out.push_back(u);
+      }
+      if (parts > 1) {
+        any = true;
+        partial_floats_ += static_cast<int64_t>(parts) * kBM * t.cols;
+        split_tiles_ += 1;
+      }
+    }
+    if (!any) return;
+    std::stable_sort(out.begin(), out.end(), [](const GemmTile& x, const GemmTile& y) { return x.kb1 - x.kb0 > y.kb1 - y.kb0; });
+    tiles_.resize(first);
+    tiles_.insert(tiles_.end(), out.begin(), out.end());
+  }
+
   int map_of(const torch::Tensor& t, int box_rows) {
     const std::array<int64_t, 5> key = {reinterpret_cast<int64_t>(t.data_ptr()), t.size(0), t.size(1), t.stride(0), box_rows};
     auto it = cache_.find(key);
@@ -361,6 +422,7 @@ class PlanBuilder {
   torch::Device device_{torch::kCPU};
   int launch_begin_ = 0;
   bool half_ = false;
+  int64_t split_tiles_ = 0, partial_floats_ = 0;
 };
 
 // `mode` as a GemmMode, checked against the operand format the plan was built for.

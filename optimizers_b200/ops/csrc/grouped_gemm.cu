@@ -20,8 +20,7 @@ constexpr int kTileBytesA = kBM * kBK * 4;  // 16 KiB
 constexpr int kTileBytesB = kBN * kBK * 4;  // 16 KiB
 constexpr int kStagePitch = 33;             // floats per staged row: conflict-free transposition
 constexpr uint32_t kIdesc = make_idesc(/*tf32*/ 2, kBM, kBN);
-constexpr uint32_t kIdescHalf = make_idesc(/*f16*/ 0, kBM, kBN);
-constexpr uint32_t kIdescHalfWide = make_idesc(/*f16*/ 0, kBM, 2 * kBN);
+constexpr uint32_t kIdescHalf = make_idesc(/*f16*/ 0, kBM, 0);  // N is filled in per tile
 
 template <int kMode>
 struct Cfg {
@@ -36,6 +35,28 @@ struct Cfg {
   // 1024 B of slack so the stage buffers can be aligned for the 128-byte swizzle.
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStagingBytes + kBarrierBytes;
 };
+
+// Partial sums of stripe q (32 rows) of one part: 32-column chunks, in each 8 groups of 4 columns by 32 rows.
+__device__ __forceinline__ float4* stripe_of(const GemmTile& tile, int part, int q) {
+  return reinterpret_cast<float4*>(tile.partial + static_cast<long long>(part) * kBM * tile.cols + q * 32 * tile.cols);
+}
+
+__device__ __forceinline__ void sum_parts(const GemmTile& tile, int q, int c, int lane, float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = 0.f;
+#pragma unroll 1
+  for (int part = 0; part < tile.parts; ++part) {
+    const float4* src = stripe_of(tile, part, q) + c * 8 * 32 + lane;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const float4 x = __ldcg(src + g * 32);
+      v[4 * g] += x.x;
+      v[4 * g + 1] += x.y;
+      v[4 * g + 2] += x.z;
+      v[4 * g + 3] += x.w;
+    }
+  }
+}
 
 // kPush: instantiation whose epilogue also stores into the peers' gather buffers; kept apart so
 // that the store loop of the common instantiation is not burdened with it.
@@ -93,8 +114,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
         const GemmTile tile = tiles[t];
         const GemmProblem* p = &problems[tile.problem];
-        const int num_kb = (p->K + kBK - 1) / kBK;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = tile.kb0; kb < tile.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
             ok = false;
             break;
@@ -127,13 +147,14 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       int it = 0;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
         const GemmTile tile = tiles[t];
-        const int num_kb = (problems[tile.problem].K + kBK - 1) / kBK;
         const int buf = it & 1;
         if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * C::kAccCols;
-        const uint32_t idesc_half = tile.cols > kBN ? kIdescHalfWide : kIdescHalf;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        // Columns beyond N are not multiplied (in steps of 16); the epilogue does not read them.
+        const int live = kHalf ? min(tile.cols, (problems[tile.problem].N - tile.n0 + 15) & ~15) : kBN;
+        const uint32_t idesc_half = kIdescHalf | (static_cast<uint32_t>(live >> 3) << 17);
+        for (int kb = tile.kb0; kb < tile.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
             ok = false;
             break;
@@ -148,7 +169,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               const uint64_t hi = static_cast<uint64_t>(k * 2), lo = static_cast<uint64_t>(4 + k * 2);
-              umma_f16(d_tmem, a_hi + lo, b_hi + hi, idesc_half, (kb | k) != 0);
+              umma_f16(d_tmem, a_hi + lo, b_hi + hi, idesc_half, kb != tile.kb0 || k != 0);
               umma_f16(d_tmem, a_hi + hi, b_hi + hi, idesc_half, 1);
               umma_f16(d_tmem, a_hi + hi, b_hi + lo, idesc_half, 1);
             }
@@ -168,11 +189,11 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
             const uint64_t koff = static_cast<uint64_t>(k * 2);
             if (kSplit) {
               // Consecutive products share one operand descriptor (b_hi, then a_hi).
-              umma_tf32(d_tmem, a_lo + koff, b_hi + koff, kIdesc, (kb | k) != 0);
+              umma_tf32(d_tmem, a_lo + koff, b_hi + koff, kIdesc, kb != tile.kb0 || k != 0);
               umma_tf32(d_tmem, a_hi + koff, b_hi + koff, kIdesc, 1);
               umma_tf32(d_tmem, a_hi + koff, b_lo + koff, kIdesc, 1);
             } else {
-              umma_tf32(d_tmem, a_hi + koff, b_hi + koff, kIdesc, (kb | k) != 0);
+              umma_tf32(d_tmem, a_hi + koff, b_hi + koff, kIdesc, kb != tile.kb0 || k != 0);
             }
           }
           umma_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
@@ -227,9 +248,31 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       // consume these products).
       const bool sym = (flags & kFlagMirror) != 0;
       const bool diag_tile = sym && tile.n0 == tile.m0;
-      if (row0 < M) {
+      const bool parted = kHalf && tile.parts > 1;
+      bool finish = row0 < M;  // this warp runs the epilogue of its stripe
+      const int chunks = kHalf ? tile.cols / 32 : kBN / 32;
+      if (parted && row0 < M) {
+        float4* own = stripe_of(tile, tile.part, q) + lane;
+        for (int c = 0; c < chunks && tile.n0 + c * 32 < N; ++c) {
+          if ((flags & kFlagPackedC) && tile.n0 + c * 32 + 31 < row0) continue;
+          float v[32];
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
+#pragma unroll
+          for (int g = 0; g < 8; ++g) own[(c * 8 + g) * 32] = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+        }
+        __threadfence();
+        __syncwarp();
+        int arrived = 0;
+        if (lane == 0) arrived = atomicAdd(tile.counter + q, 1);
+        finish = __shfl_sync(0xffffffffu, arrived, 0) == tile.parts - 1;
+        if (finish) {
+          if (lane == 0) tile.counter[q] = 0;
+          __threadfence();
+        }
+      }
+      if (finish) {
 #pragma unroll 1
-        for (int c = 0; c < (kHalf ? tile.cols / 32 : kBN / 32); ++c) {
+        for (int c = 0; c < chunks; ++c) {
           const int col0 = tile.n0 + c * 32;
           if (col0 >= N) break;
           if ((flags & kFlagPackedC) && col0 + 31 < row0) continue;  // chunk strictly below the diagonal
@@ -237,7 +280,11 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           const bool mirror = sym && (!diag_tile || c > q);
           const bool diag_chunk = diag_tile && c == q;
           float v[32];
-          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
+          if (kHalf && parted) {
+            sum_parts(tile, q, c, lane, v);
+          } else {
+            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
+          }
           float sq_chunk = 0.f;
           if constexpr (kHalf) {
 #pragma unroll

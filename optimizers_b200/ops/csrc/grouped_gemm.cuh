@@ -97,11 +97,19 @@ struct PeerPush {
   int dtype;      // 0 fp32, 1 bf16, 2 fp16
 };
 
-struct GemmTile {
+// One work item: an output tile, or with parts > 1 the share [kb0, kb1) of its K blocks.  Every part leaves its
+// accumulator at `partial` (part-major, kBM x cols floats each); of each 32-row stripe the warp that arrives
+// last at counter[stripe] adds the parts up in their order, so that the result does not depend on the
+// arrival, and runs the epilogue on the sum.  No part waits for another.
+struct alignas(16) GemmTile {
   int problem;
   int m0;  // first row of the tile
   int n0;  // first column of the tile
   int cols;  // 128, or 256 (kGemmHalfPair only)
+  int kb0, kb1;
+  int part, parts;
+  float* partial;
+  int* counter;  // [kBM / 32], zero between launches
 };
 
 enum GemmMode : int { kGemmTf32 = 0, kGemmTf32x3 = 1, kGemmHalfPair = 2 };
