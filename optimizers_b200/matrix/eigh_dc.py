@@ -79,6 +79,7 @@ LEAF = 128  # largest problem the Jacobi kernel takes
 _MAX_ATTEMPTS = 3  # sign computations per subproblem before its root is given up
 _MAX_ROUNDS = 40  # rounds of the work list before the remaining roots are given up
 _IDEMPOTENCY_TOL = 0.05  # bound on |trace(P) - ||P||_F^2| = |sum p (1 - p)| over the eigenvalues p of P
+_SIGN_BOUND = 8.0  # of the entries of X, X^2 and W in the sign iteration (their spectra stay below 4)
 _NUDGE = 3e-5  # relative shift of the split point for a repeated sign computation
 
 
@@ -557,6 +558,9 @@ class NativeBackend:
 
     def sign_projector(self, subs: list[Sub]) -> None:
         ext, dev = self.ext, self.device
+        if dev.type == "cuda":  # (the stand-in of the extension on a CPU has fp32 operands)
+            self._sign_projector_on_pairs(subs)
+            return
         start = _mats(ext, dev, [(s.n, s.n) for s in subs], plain=False)
         table = ext.build_sym_table(
             [(s.A.plain, start[i].hi, start[i].lo, None, 1.0 / s.spread, -s.sigma / s.spread) for i, s in enumerate(subs)]
@@ -622,6 +626,89 @@ class NativeBackend:
             s.rank = int(round(fro2)) if finite else -1
             s.idem_err = trace - fro2 if finite else float("nan")
         return [X[cur][i] for i in idx]
+
+    def _sign_projector_on_pairs(self, subs: list[Sub]) -> None:
+        """``sign_projector`` with the iteration's matrices as scaled fp16 pairs: twice the tf32 rate and half the
+        operand bytes, with the smaller accumulation error.  Every matrix of the iteration is a polynomial in
+        X whose spectrum the schedule keeps within a few units, and no entry exceeds the spectral norm:
+        one bound serves them all.  The projector leaves as the tf32 pair its readers take."""
+        ext, dev = self.ext, self.device
+        bound = torch.tensor([_SIGN_BOUND, 0.0], device=dev)
+        sizes = [s.n for s in subs]
+
+        def start(sources, scales, todo):
+            plain = _mats(ext, dev, [(s.n, s.n) for s in todo], pair=False)
+            ext.shift_scale_split(*ext.build_sym_table(
+                [(src, m.plain, None, None, a, b) for src, m, (a, b) in zip(sources, plain, scales, strict=True)]
+            ))
+            pairs = ext.alloc_pair_batch([s.n for s in todo], dev)
+            metas = torch.zeros(len(todo), 2, device=dev)
+            ext.pair_mirrors(*ext.build_pair_table([(m.plain, x, None, metas[i]) for i, (m, x) in enumerate(zip(plain, pairs, strict=True))]))
+            return pairs, list(metas)
+
+        todo = list(subs)
+        X0 = start([s.A.plain for s in subs], [(1.0 / s.spread, -s.sigma / s.spread) for s in subs], subs)
+        for stage, schedule in enumerate(SIGN_STAGES):
+            projectors = self._sign_stage_on_pairs(todo, *X0, schedule, bound)
+            self.sign_stages_run[stage] += len(todo)
+            again = []
+            for s, P in zip(todo, projectors, strict=True):
+                s.extra["P"] = P
+                if stage + 1 < len(SIGN_STAGES) and s.rank >= 0 and not abs(s.idem_err) <= _IDEMPOTENCY_TOL:
+                    again.append(s)
+            if not again:
+                break
+            # not projectors yet: X = 2 P - I goes through the next stage (an elementwise pass)
+            sums = torch._foreach_add([s.extra["P"].hi for s in again], [s.extra["P"].lo for s in again])
+            todo, X0 = again, start(sums, [(2.0, -1.0)] * len(again), again)
+
+    def _sign_stage_on_pairs(self, subs: list[Sub], X0: list[Tensor], metas: list[Tensor], schedule: tuple, bound: Tensor) -> list[_Mat]:
+        ext, dev, F = self.ext, self.device, self.ext
+        sizes, idx = [s.n for s in subs], range(len(subs))
+        X = [X0, ext.alloc_pair_batch(sizes, dev), ext.alloc_pair_batch(sizes, dev)]  # the start (own bounds), then in turn
+        Y, W = ext.alloc_pair_batch(sizes, dev), ext.alloc_pair_batch(sizes, dev)
+        Yp = [m.plain for m in _mats(ext, dev, [(n, n) for n in sizes], pair=False)]
+        stats = torch.zeros(len(subs), 2, device=dev)
+        sym = F.FLAG_MIRROR | F.FLAG_SPLIT_OUT | F.FLAG_FIXED_SCALE
+
+        def spec(a, b, a_meta, b_meta, out, c, flags):
+            c_ld = 0 if c is None else c.stride(0)
+            return (a, None, b, None, c, out, None, None, c_ld, out.stride(0), flags | sym | (F.FLAG_NO_C if c is None else 0), True,
+                    None, None, (a_meta, b_meta, bound))
+
+        plans = {}
+        # W = c Y Y + b Y + a I: beta applies to the plain copy of Y that C holds
+        second = ext.build_gemm_plan([spec(Y[i], Y[i], bound, bound, W[i], Yp[i], F.FLAG_ADD_DIAG) for i in idx])
+        meta = lambda cur, i: metas[i] if cur == 0 else bound  # noqa: E731
+        cur, last = 0, len(schedule) - 1
+        for it, (a, b, c) in enumerate(schedule):
+            nxt = 1 if cur != 1 else 2
+            if cur not in plans:
+                plans[cur] = (
+                    ext.build_gemm_plan([spec(X[cur][i], X[cur][i], meta(cur, i), meta(cur, i), Y[i], Yp[i], 0) for i in idx]),
+                    ext.build_gemm_plan([spec(X[cur][i], W[i], meta(cur, i), bound, X[nxt][i], None, 0) for i in idx]) if it != last else None,
+                )
+            first, third = plans[cur]
+            ext.run_gemm_plan(*first, 1.0, 0.0, F.HALF_PAIR_SYM, self.status)
+            ext.run_gemm_plan(*second, c, b, F.HALF_PAIR_SYM, self.status, a)
+            if it == last:
+                # P = X W / 2 + I / 2 with ||P||_F^2 and trace(P) from the epilogue
+                out = _mats(ext, dev, [(n, n) for n in sizes], plain=False)
+                flags = F.FLAG_MIRROR | F.FLAG_SPLIT_OUT | F.FLAG_NO_C | F.FLAG_ADD_DIAG | F.FLAG_SUMSQ | F.FLAG_TRACE
+                final = [
+                    (X[cur][i], None, W[i], None, None, out[i].hi, out[i].lo, stats[i], 0, out[i].hi.stride(0), flags, True,
+                     None, None, (meta(cur, i), bound, None))
+                    for i in idx
+                ]
+                ext.run_gemm_plan(*ext.build_gemm_plan(final), 0.5, 0.0, F.HALF_PAIR_SYM, self.status, 0.5)
+            else:
+                ext.run_gemm_plan(*third, 1.0, 0.0, F.HALF_PAIR_SYM, self.status)
+            cur = nxt
+        for s, (fro2, trace) in zip(subs, stats.cpu().tolist(), strict=True):
+            finite = fro2 == fro2 and abs(fro2) != float("inf")
+            s.rank = int(round(fro2)) if finite else -1
+            s.idem_err = trace - fro2 if finite else float("nan")
+        return out
 
     def split_basis(self, subs: list[Sub]) -> None:
         ext, dev = self.ext, self.device

@@ -224,15 +224,19 @@ class PlanBuilder {
     p.b_meta = q.b_meta;
     p.d_meta = q.d_meta;
     const bool half = p.a_meta != nullptr;
-    TORCH_CHECK(problems_.empty() || half == half_, "a plan holds one operand format");
+    const bool half_sym = half && (p.flags & (kFlagMirror | kFlagFixedScale)) != 0;
+    TORCH_CHECK(problems_.empty() || (half == half_ && half_sym == half_sym_), "a plan holds one operand format");
     half_ = half;
+    half_sym_ = half_sym;
     if (half) {
       TORCH_CHECK(p.b_meta != nullptr, "both operands of a half-pair product need their meta data");
       TORCH_CHECK(q.K % kBK == 0, "half-pair operands are padded to a multiple of ", kBK, " along K");
-      TORCH_CHECK(!(p.flags & kFlagMirror), "mirrored output has no half-pair form");
-      if (p.flags & kFlagSplitOut) {
-        TORCH_CHECK((p.flags & kFlagNoC) && !(p.flags & (kFlagSumSq | kFlagTrace | kFlagAddDiag | kFlagPackedC)),
-                    "a half-pair split output stands alone");
+      TORCH_CHECK(half_sym || !(p.flags & kFlagSplitOut) || p.d_lo == nullptr, "a tf32 pair from half pairs needs a symmetric plan");
+      if ((p.flags & kFlagSplitOut) && p.d_lo == nullptr) {  // (with a d_lo the output is a tf32 pair)
+        TORCH_CHECK(!(p.flags & (kFlagPackedC | kFlagSquareAcc | kFlagPeerPush)), "this epilogue has no half-pair form");
+        TORCH_CHECK(!half_sym || (p.flags & kFlagFixedScale), "a symmetric plan's half-pair outputs have a given bound");
+        TORCH_CHECK(half_sym || ((p.flags & kFlagNoC) && !(p.flags & (kFlagSumSq | kFlagTrace | kFlagAddDiag))),
+                    "a half-pair split output that is more than alpha A B^T needs a symmetric plan");
         TORCH_CHECK(p.d_hi != nullptr && p.d_meta != nullptr && p.ldd % kBK == 0 && p.ldd >= p.N &&
                         reinterpret_cast<uintptr_t>(p.d_hi) % 16 == 0,
                     "a half-pair split output needs its meta data, a 16-byte aligned base and a pitch that is a multiple of ", kBK);
@@ -309,7 +313,7 @@ class PlanBuilder {
         }
       }
     }
-    if (half_) split_along_k(first);
+    if (half_ && !half_sym_) split_along_k(first);
     launch_begin_ = static_cast<int>(problems_.size());
     return {first, static_cast<int64_t>(tiles_.size()) - first};
   }
@@ -349,8 +353,8 @@ class PlanBuilder {
       t.counter = reinterpret_cast<int*>(base + table_bytes + map_bytes) + reinterpret_cast<uintptr_t>(t.counter);
     }
     auto d_tiles = upload_bytes(tiles_.data(), tiles_.size() * sizeof(GemmTile), device_);
-    // The element type of the tile list tells a half-pair plan from an fp32 one (gemm_mode below).
-    return {buffer, half_ ? d_tiles.view(torch::kInt32) : d_tiles};
+    // The element type of the tile list tells which modes a plan may run in (gemm_mode below).
+    return {buffer, half_sym_ ? d_tiles.view(torch::kInt16) : half_ ? d_tiles.view(torch::kInt32) : d_tiles};
   }
 
  private:
@@ -368,8 +372,8 @@ class PlanBuilder {
   // Where a launch has too few tiles for the SMs, or single tiles with a K loop far longer than the others', the long
   // loops are cut into parts of about an SM's share of all K blocks, of at least kMinPart blocks (a part
   // costs a round trip of its accumulator through the L2, a few microseconds, as much as about 8 blocks) and
-  // at most kMaxParts (the last to arrive reads them all).  On one B200 the four launches of a step over ResNet
-  // weights, among them the Gram of a 3 x 98304 unfolding, went from 387 to 77 us.
+  // at most kMaxParts (the last to arrive reads them all).  On one B200 a step over ResNet weights, among
+  // them the Gram of a 3 x 98304 unfolding, went from 517 to 194 us.
   void split_along_k(int64_t first) {
     constexpr int kMinPart = 12, kMaxParts = 32;
     const int sms = at::cuda::getDeviceProperties(device_.index())->multiProcessorCount;
@@ -421,14 +425,16 @@ class PlanBuilder {
   std::map<std::array<int64_t, 5>, int> cache_;
   torch::Device device_{torch::kCPU};
   int launch_begin_ = 0;
-  bool half_ = false;
+  bool half_ = false, half_sym_ = false;
   int64_t split_tiles_ = 0, partial_floats_ = 0;
 };
 
 // `mode` as a GemmMode, checked against the operand format the plan was built for.
 GemmMode gemm_mode(int64_t mode, const torch::Tensor& tiles) {
-  TORCH_CHECK(mode >= kGemmTf32 && mode <= kGemmHalfPair, "unknown GEMM mode ", mode);
-  TORCH_CHECK((mode == kGemmHalfPair) == (tiles.scalar_type() == torch::kInt32), "GEMM mode and operand format of the plan differ");
+  TORCH_CHECK(mode >= kGemmTf32 && mode <= kGemmHalfPairSym, "unknown GEMM mode ", mode);
+  TORCH_CHECK((mode == kGemmHalfPair) == (tiles.scalar_type() == torch::kInt32) &&
+                  (mode == kGemmHalfPairSym) == (tiles.scalar_type() == torch::kInt16),
+              "GEMM mode and operand format of the plan differ");
   return static_cast<GemmMode>(mode);
 }
 
@@ -1209,6 +1215,22 @@ alloc_mat_batch(const std::vector<int64_t>& rows, const std::vector<int64_t>& co
   return out;
 }
 
+// The square half-pair arrays of a batch, [n, pad32(n)] each, as views of one allocation.
+std::vector<torch::Tensor> alloc_pair_batch(const std::vector<int64_t>& sizes, const torch::Device& device) {
+  int64_t total = 0;
+  for (const int64_t n : sizes) total += n * ((n + kBK - 1) / kBK * kBK);
+  auto block = torch::empty({std::max<int64_t>(total, 1)}, torch::TensorOptions().dtype(torch::kFloat32).device(device));
+  std::vector<torch::Tensor> out;
+  out.reserve(sizes.size());
+  int64_t offset = 0;
+  for (const int64_t n : sizes) {
+    const int64_t ld = (n + kBK - 1) / kBK * kBK;
+    out.push_back(block.as_strided({n, ld}, {ld, 1}, offset));
+    offset += n * ld;
+  }
+  return out;
+}
+
 // Table for the per-matrix passes of the eigensolver.  Each spec: (src, dst_hi | None, dst_lo | None,
 // stats | None, a, b).
 std::tuple<torch::Tensor, torch::Tensor, int64_t> build_sym_table(const std::vector<py::tuple>& specs) {
@@ -1499,6 +1521,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("householder_qr", &householder_qr);
   m.attr("QR_PANEL") = kQrPanel;
   m.def("alloc_mat_batch", &alloc_mat_batch);
+  m.def("alloc_pair_batch", &alloc_pair_batch);
+  m.attr("FLAG_FIXED_SCALE") = kFlagFixedScale;
   m.def("build_sym_table", &build_sym_table);
   m.def("sym_measure", &sym_measure);
   m.def("sq_offdiag", &sq_offdiag);
@@ -1510,6 +1534,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("build_transpose_table", &build_transpose_table);
   m.def("transpose_split", &transpose_split);
   m.attr("HALF_PAIR") = static_cast<int>(kGemmHalfPair);
+  m.attr("HALF_PAIR_SYM") = static_cast<int>(kGemmHalfPairSym);
   static_assert(static_cast<int>(kGemmHalfPair) == static_cast<int>(kFormPair), "one code names the operand format");
   m.def("build_pair_table", &build_pair_table);
   m.def("pair_mirrors", &pair_mirrors);

@@ -24,12 +24,13 @@ constexpr uint32_t kIdescHalf = make_idesc(/*f16*/ 0, kBM, 0);  // N is filled i
 
 template <int kMode>
 struct Cfg {
-  static constexpr int kAccCols = kMode == kGemmHalfPair ? 2 * kBN : kBN;  // columns of one accumulator buffer
+  static constexpr bool kHalf = kMode == kGemmHalfPair || kMode == kGemmHalfPairSym;
+  static constexpr int kAccCols = kHalf ? 2 * kBN : kBN;  // columns of one accumulator buffer
   static constexpr int kTmemCols = 2 * kAccCols;                           // two accumulator buffers
   // tf32x3: hi and lo of both operands; half pairs: one A tile and up to two B tiles (256 columns)
   static constexpr int kStageBytes =
-      kMode == kGemmTf32x3 ? 2 * (kTileBytesA + kTileBytesB) : kTileBytesA + (kMode == kGemmHalfPair ? 2 : 1) * kTileBytesB;
-  static constexpr int kStages = kMode == kGemmTf32x3 ? 3 : kMode == kGemmHalfPair ? 4 : 6;
+      kMode == kGemmTf32x3 ? 2 * (kTileBytesA + kTileBytesB) : kTileBytesA + (kHalf ? 2 : 1) * kTileBytesB;
+  static constexpr int kStages = kMode == kGemmTf32x3 ? 3 : kHalf ? 4 : 6;
   static constexpr int kStagingBytes = kEpilogueWarps * 32 * kStagePitch * 4;
   static constexpr int kBarrierBytes = 256;
   // 1024 B of slack so the stage buffers can be aligned for the 128-byte swizzle.
@@ -58,6 +59,81 @@ __device__ __forceinline__ void sum_parts(const GemmTile& tile, int q, int c, in
   }
 }
 
+// Epilogue of one 32 x 32 chunk whose result is stored as half pairs: thread `lane` holds row row0 + lane and owns
+// its 128-byte chunk (zero beyond N, which the next product reads as K padding).  The transposed copy of a symmetric
+// result goes through the staging tile, after which a thread owns a row of the transpose.
+__device__ __forceinline__ void half_pair_chunk(float (&v)[32], float* st, float* __restrict__ Cp, float* __restrict__ Dhi, int M,
+                                                int N, int ldc, int ldd, int flags, int row0, int col0, int lane, float alpha,
+                                                float beta, float gamma, float scale, bool mirror, bool diag_chunk, float& sq,
+                                                float& tr) {
+  const int row = row0 + lane;
+  const bool live = row < M, write_c = !(flags & kFlagNoC);
+  float* crow = write_c ? Cp + static_cast<long long>(row) * ldc + col0 : nullptr;
+  const bool vec = write_c && col0 + 32 <= N && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(Cp) & 15) == 0;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    float old[4] = {0.f, 0.f, 0.f, 0.f};
+    if (write_c && beta != 0.f && live) {
+      if (vec) {
+        const float4 o = reinterpret_cast<const float4*>(crow)[g];
+        old[0] = o.x; old[1] = o.y; old[2] = o.z; old[3] = o.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) old[k] = col0 + 4 * g + k < N ? crow[4 * g + k] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = 4 * g + k;
+      float x = alpha * v[j] + (write_c && beta != 0.f ? beta * old[k] : 0.f);
+      if ((flags & kFlagAddDiag) && col0 + j == row) x += gamma;
+      v[j] = live && col0 + j < N ? x : 0.f;
+      if ((flags & kFlagTrace) && col0 + j == row) tr += v[j];
+    }
+  }
+  if (mirror || diag_chunk) {
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) st[lane * kStagePitch + j] = v[j];
+    __syncwarp();
+  }
+  if (diag_chunk) {  // symmetric bit for bit: entries below the diagonal are those above it
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = j >= lane ? v[j] : st[j * kStagePitch + lane];
+  }
+  if (flags & kFlagSumSq) {
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) s = fmaf(v[j], v[j], s);
+    sq += mirror ? 2.f * s : s;
+  }
+  auto store_c = [&](float* dst, int count, bool v4) {
+    if (v4) {
+#pragma unroll
+      for (int g = 0; g < 8; ++g) reinterpret_cast<float4*>(dst)[g] = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < count) dst[j] = v[j];
+    }
+  };
+  if (live) {
+    if (write_c) store_c(crow, N - col0, vec);
+    store_pair_chunk(Dhi + static_cast<long long>(row) * ldd + col0, v, scale);
+  }
+  if (mirror) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = st[i * kStagePitch + lane];
+    const int trow = col0 + lane;
+    if (trow < N) {
+      const bool tvec = row0 + 32 <= M && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(Cp) & 15) == 0;
+      if (write_c) store_c(Cp + static_cast<long long>(trow) * ldc + row0, M - row0, tvec);
+      store_pair_chunk(Dhi + static_cast<long long>(trow) * ldd + row0, v, scale);
+    }
+    __syncwarp();
+  }
+}
+
 // kPush: instantiation whose epilogue also stores into the peers' gather buffers; kept apart so
 // that the store loop of the common instantiation is not burdened with it.
 template <int kMode, bool kPush>
@@ -66,7 +142,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
                     float alpha, float beta, float gamma, int* __restrict__ status, const PeerPush push) {
   using C = Cfg<kMode>;
   constexpr int kStages = C::kStages;
-  constexpr bool kSplit = kMode == kGemmTf32x3, kHalf = kMode == kGemmHalfPair;
+  constexpr bool kSplit = kMode == kGemmTf32x3, kHalf = C::kHalf, kSym = kMode == kGemmHalfPairSym;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -232,7 +308,9 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       if constexpr (kHalf) {
         inv_a = pair_inverse_scale(p->a_meta[0]);
         inv_b = pair_inverse_scale(p->b_meta[0]);
-        if (flags & kFlagSplitOut) {
+        if (kSym && (flags & kFlagSplitOut) && (flags & kFlagFixedScale)) {
+          scale_d = pair_scale(p->d_meta[0]);
+        } else if ((flags & kFlagSplitOut) && Dlo == nullptr) {
           const float bound = fabsf(alpha) * pair_row_bound(p->a_meta, p->K) * pair_row_bound(p->b_meta, p->K);
           scale_d = pair_scale(bound);
           if (threadIdx.x == 64) {
@@ -246,9 +324,9 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       // the chunks on the diagonal are symmetrised, so the stored matrix is symmetric bit for bit
       // (an antisymmetric rounding residue would be amplified by the polynomial iterations that
       // consume these products).
-      const bool sym = (flags & kFlagMirror) != 0;
+      const bool sym = kMode != kGemmHalfPair && (flags & kFlagMirror) != 0;
       const bool diag_tile = sym && tile.n0 == tile.m0;
-      const bool parted = kHalf && tile.parts > 1;
+      const bool parted = kMode == kGemmHalfPair && tile.parts > 1;
       bool finish = row0 < M;  // this warp runs the epilogue of its stripe
       const int chunks = kHalf ? tile.cols / 32 : kBN / 32;
       if (parted && row0 < M) {
@@ -280,7 +358,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           const bool mirror = sym && (!diag_tile || c > q);
           const bool diag_chunk = diag_tile && c == q;
           float v[32];
-          if (kHalf && parted) {
+          if (kMode == kGemmHalfPair && parted) {
             sum_parts(tile, q, c, lane, v);
           } else {
             tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
@@ -289,7 +367,7 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           if constexpr (kHalf) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = (v[j] * inv_a) * inv_b;
-            if (flags & kFlagSplitOut) {
+            if (!kSym && (flags & kFlagSplitOut)) {
               // One thread owns the 128-byte chunk of its row: 32 hi, then 32 lo (zero beyond N, which
               // the next product reads as K padding).
               if (row0 + lane < M) {
@@ -297,6 +375,11 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
                 for (int j = 0; j < 32; ++j) v[j] = col0 + j < N ? alpha * v[j] : 0.f;
                 store_pair_chunk(Dhi + static_cast<long long>(row0 + lane) * ldd + col0, v, scale_d);
               }
+              continue;
+            }
+            if (kSym && (flags & kFlagSplitOut) && Dlo == nullptr) {
+              half_pair_chunk(v, st, Cp, Dhi, M, N, ldc, ldd, flags, row0, col0, lane, alpha, beta, gamma, scale_d, mirror,
+                              diag_chunk, sq, tr);
               continue;
             }
           }
@@ -553,6 +636,8 @@ void launch_grouped_gemm(const GemmProblem* problems, const GemmTile* tiles, int
   auto go = [&](auto launch) { launch(problems, tiles, num_tiles, alpha, beta, gamma, status, max_ctas, stream, pp); };
   if (mode == kGemmHalfPair) {
     pushing ? go(launch_impl<kGemmHalfPair, true>) : go(launch_impl<kGemmHalfPair, false>);
+  } else if (mode == kGemmHalfPairSym) {
+    go(launch_impl<kGemmHalfPairSym, false>);
   } else if (mode == kGemmTf32x3) {
     pushing ? go(launch_impl<kGemmTf32x3, true>) : go(launch_impl<kGemmTf32x3, false>);
   } else {

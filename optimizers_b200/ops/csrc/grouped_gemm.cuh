@@ -62,6 +62,9 @@ constexpr int kFlagPeerPush = 32;   // also store the result, cast to the commun
                                     // all-gather of the search directions happens tile by tile from
                                     // the epilogue of the GEMM that produces them
 
+constexpr int kFlagFixedScale = 512;  // half-pair split output: the caller has set the bound in d_meta; needed where
+                                      // the result is more than alpha A B^T
+
 constexpr int kErrPipelineTimeout = 1;  // a bounded mbarrier wait expired
 
 struct alignas(128) GemmProblem {
@@ -112,7 +115,10 @@ struct alignas(16) GemmTile {
   int* counter;  // [kBM / 32], zero between launches
 };
 
-enum GemmMode : int { kGemmTf32 = 0, kGemmTf32x3 = 1, kGemmHalfPair = 2 };
+// kGemmHalfPairSym: kGemmHalfPair with the epilogues of the symmetric iterations (split outputs with a given bound,
+// mirrored, with beta, diagonal, norm and trace); an instantiation of its own, so that their registers do
+// not weigh on the step's products.
+enum GemmMode : int { kGemmTf32 = 0, kGemmTf32x3 = 1, kGemmHalfPair = 2, kGemmHalfPairSym = 3 };
 
 constexpr int kBM = 128;
 constexpr int kBN = 128;

@@ -20,7 +20,7 @@ def _pad(n):
 
 
 def _scale(meta):
-    return 2.0 ** (14 - torch.floor(torch.log2(meta[0].double()))).clamp(-110, 110)
+    return 2.0 ** (15.0 - torch.frexp(meta[0])[1].double()).clamp(-110, 110)
 
 
 def _pairs(x):
@@ -115,6 +115,42 @@ def test_mirrors_are_converted_in_place(ext, d, scale):
     assert float(meta[0]) == float(X.abs().max())
     for got, want in ((buf, X), (t, X.T)):  # 22 bits, or 2^-25 steps of the scaled value
         assert bool(((_value(got, meta, d) - want.double()).abs() <= 2.0**-22 * want.abs() + 2.0**-25 / _scale(meta)).all())
+
+
+# The epilogues of the symmetric iterations: one tile, ragged edges, several tiles, wide tiles.
+@pytest.mark.parametrize("sizes", [(1,), (33, 128), (200, 300, 31), (1500, 1500)])
+def test_symmetric_products_on_pairs(ext, sizes):
+    gen = torch.Generator(device="cuda").manual_seed(sum(sizes))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    bound = torch.tensor([8.0, 0.0], device="cuda")
+    specs, finals, checks = [], [], []
+    stats = torch.zeros(len(sizes), 2, device="cuda")
+    for i, n in enumerate(sizes):
+        X = torch.randn(n, n, device="cuda", generator=gen)
+        X = (X + X.T) / (2.0 * n**0.5)
+        x, meta = _pairs(X)
+        c = torch.randn(n, n, device="cuda", generator=gen) / n**0.5
+        c = (c + c.T) / 2
+        d = torch.full((n, _pad(n)), float("nan"), device="cuda")
+        pitch = (n + 3) // 4 * 4
+        hi, lo = (torch.full((n, pitch), float("nan"), device="cuda") for _ in range(2))
+        XX = X.double() @ X.double().T
+        checks.append((c, d, hi, lo, 2.0 * XX - 0.5 * c.double() + 0.7 * torch.eye(n, device="cuda"), 0.5 * XX + 0.5 * torch.eye(n, device="cuda"), n))
+        sym = ext.FLAG_MIRROR | ext.FLAG_SPLIT_OUT | ext.FLAG_ADD_DIAG
+        specs.append((x, None, x, None, c, d, None, None, c.stride(0), d.stride(0), sym | ext.FLAG_FIXED_SCALE, True, None, None, (meta, meta, bound)))
+        finals.append((x, None, x, None, None, hi, lo, stats[i], 0, pitch, sym | ext.FLAG_NO_C | ext.FLAG_SUMSQ | ext.FLAG_TRACE, True,
+                       None, None, (meta, meta, None)))
+    ext.run_gemm_plan(*ext.build_gemm_plan(specs), 2.0, -0.5, ext.HALF_PAIR_SYM, status, 0.7)
+    ext.run_gemm_plan(*ext.build_gemm_plan(finals), 0.5, 0.0, ext.HALF_PAIR_SYM, status, 0.5)
+    for i, (c, d, hi, lo, want, proj, n) in enumerate(checks):
+        tol = _bound(n) + 2.0**-22
+        value, split = _value(d, bound, n), hi[:, :n].double() + lo[:, :n].double()
+        for got, ref in ((c.double(), want), (value, want), (split, proj)):
+            assert float((got - ref).norm() / ref.norm()) < tol
+            assert torch.equal(got, got.T)
+        assert abs(float(stats[i, 0]) / float((proj**2).sum()) - 1) < 2 * tol + 1e-5
+        assert abs(float(stats[i, 1]) - float(torch.trace(proj))) < (tol + 1e-5) * float(proj.norm()) * n**0.5
+    assert int(status) == 0
 
 
 def test_plans_of_one_format_are_not_run_in_another(ext):
