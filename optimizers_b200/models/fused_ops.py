@@ -95,10 +95,19 @@ class _LMHeadXent(torch.autograd.Function):
         scale = (grad_out / valid).to(torch.float32)
         dx = dw = None
         if ctx.needs_input_grad[0]:
-            dx = (torch.mm(dlogits, wb) * scale).to(ctx.x_dtype)
+            dx = _scaled(torch.mm(dlogits, wb), scale, ctx.x_dtype)
         if ctx.needs_input_grad[1]:
-            dw = (torch.mm(dlogits.t(), xb)[: ctx.V] * scale).to(ctx.w_dtype)
+            dw = _scaled(torch.mm(dlogits.t(), xb)[: ctx.V], scale, ctx.w_dtype)
         return dx, dw, None, None
+
+
+def _scaled(product: Tensor, scale: Tensor, dtype: torch.dtype) -> Tensor:
+    """``scale`` times a bf16 product in ``dtype`` (fp32 without a rounding to bf16 in between).  A backward
+    that is itself recorded (``create_graph``) keeps to differentiable operations."""
+    if dtype not in (torch.float32, torch.bfloat16) or torch.is_grad_enabled():
+        return (product * scale).to(dtype)
+    _count()
+    return _ext().scale_cast(product, scale, dtype == torch.bfloat16)
 
 
 def lm_head_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, ignore_index: int = -100) -> Tensor:
