@@ -1092,13 +1092,14 @@ class NativeGroupEngine:
             g_bc2 = float(glist._bias_correction2)
         l2 = weight_decay if (weight_decay_type == WeightDecayType.L2) else 0.0
 
-        self._step_scratch.zero_()
+        if not self._half:
+            self._step_scratch.zero_()
         blocks_t, tiles_t, n_tiles = self._table
         ext.grad_prologue(
             blocks_t, tiles_t, n_tiles, self._grad_ptrs_dev, l2, beta1, beta3, bc1, self._graft_kind,
             g_beta2, g_weight, g_bc2, g_eps, self._form, self._status,
             self._arena.world if self._pull else 0, 1.0 / self._arena.world if self._pull else 1.0,
-            *((graft_only,) if self._half else ()),
+            *((graft_only, self._step_scratch) if self._half else ()),
         )
         launches += 3 if self._half else 2
         self._mark("grad_prologue")

@@ -645,9 +645,13 @@ void grad_prologue(const torch::Tensor& blocks, const torch::Tensor& tiles, int6
                    const torch::Tensor& grad_ptrs, double l2_weight_decay, double beta1, double beta3,
                    double bias_correction1, int64_t graft_kind, double graft_beta2, double graft_weight,
                    double graft_bc2, double graft_eps, int64_t write_split, torch::Tensor status,
-                   int64_t num_grad_peers, double grad_scale, bool filtered_plain) {
+                   int64_t num_grad_peers, double grad_scale, bool filtered_plain, const std::optional<torch::Tensor>& scratch) {
   LaunchScope scope("ob200::grad_prologue");
   c10::cuda::CUDAGuard guard(blocks.device());
+  if (scratch.has_value()) {  // the norms and meta data the step accumulates into start at zero
+    TORCH_CHECK(scratch->is_cuda() && scratch->is_contiguous(), "step scratch must be a contiguous CUDA tensor");
+    C10_CUDA_CHECK(cudaMemsetAsync(scratch->data_ptr(), 0, scratch->nbytes(), at::cuda::getCurrentCUDAStream()));
+  }
   PrologueArgs a;
   a.blocks = reinterpret_cast<const BlockDesc*>(blocks.data_ptr());
   a.tiles = tile_ptr(tiles);
@@ -1546,7 +1550,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("grad_prologue", &grad_prologue, py::arg("blocks"), py::arg("tiles"), py::arg("num_tiles"), py::arg("grad_ptrs"),
         py::arg("l2_weight_decay"), py::arg("beta1"), py::arg("beta3"), py::arg("bias_correction1"), py::arg("graft_kind"),
         py::arg("graft_beta2"), py::arg("graft_weight"), py::arg("graft_bc2"), py::arg("graft_eps"), py::arg("write_split"),
-        py::arg("status"), py::arg("num_grad_peers"), py::arg("grad_scale"), py::arg("filtered_plain") = false);
+        py::arg("status"), py::arg("num_grad_peers"), py::arg("grad_scale"), py::arg("filtered_plain") = false, py::arg("scratch") = std::optional<torch::Tensor>());
   m.def("direction_epilogue", &direction_epilogue);
   m.def("gathered_apply", &gathered_apply);
   m.def("peer_barrier", &peer_barrier);

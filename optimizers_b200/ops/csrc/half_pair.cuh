@@ -17,11 +17,11 @@ namespace ob200 {
 
 constexpr int kPairChunk = 32;  // elements of one chunk
 
-// Exponent field of the scale for bound B, held within 2^-110 .. 2^110.
+// Exponent field of the scale for bound B: 13 at the largest B (or an overflowed one), at most 2^110.
 __device__ __forceinline__ int pair_scale_field(float bound) {
   const int e = static_cast<int>((__float_as_uint(bound) >> 23) & 255u);  // 255: B overflowed
   const int f = bound == 0.f ? 127 : 127 + 14 + 127 - e;
-  return f < 17 ? 17 : f > 237 ? 237 : f;
+  return f > 237 ? 237 : f;
 }
 
 __device__ __forceinline__ float pair_scale(float bound) {

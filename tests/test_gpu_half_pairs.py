@@ -20,7 +20,7 @@ def _pad(n):
 
 
 def _scale(meta):
-    return 2.0 ** (15.0 - torch.frexp(meta[0])[1].double()).clamp(-110, 110)
+    return 2.0 ** (15.0 - torch.frexp(meta[0])[1].double()).clamp(max=110)
 
 
 def _pairs(x):
@@ -104,7 +104,7 @@ def test_gram_of_pairs_in_the_packed_triangle(ext, d, K):
 
 
 @pytest.mark.parametrize("d", [1, 31, 32, 33, 200])
-@pytest.mark.parametrize("scale", [1e-30, 1.0, 1e30])
+@pytest.mark.parametrize("scale", [1e-30, 1.0, 1e37])
 def test_mirrors_are_converted_in_place(ext, d, scale):
     gen = torch.Generator(device="cuda").manual_seed(d)
     X = torch.randn(d, d, device="cuda", generator=gen) * scale
