@@ -4,7 +4,7 @@ The torch step walks Python lists of per-block tensors and launches several kern
 The native engine instead keeps a *device block table* for the group and runs the whole step as
 a fixed, short sequence of grouped launches:
 
-    grad_prologue        one pass over the gradients (L2, tf32 operand splits in both
+    grad_prologue        the gradients' largest entries, then one pass over them (L2, operand forms in both
                          orientations, filtered-gradient EMA, grafting second moment and norm)
     grouped SYRK         every factor of every block:  F <- beta2 F + w X X^T, written straight
                          into the (packed) factor state by the tensor-core kernel's epilogue
@@ -971,7 +971,7 @@ class NativeGroupEngine:
         direction in the place of G, chain intermediates in the place of G^T) are counted once.
 
         ``state``: what a checkpoint holds (factors, inverse roots / eigenvectors, corrected
-        eigenvalues, filtered gradient, grafting and momentum buffers).  ``operands``: the tf32
+        eigenvalues, filtered gradient, grafting and momentum buffers).  ``operands``: the
         (hi, lo) operand arrays of the gradient, its transpose, the filtered gradient and the chain
         intermediates.  ``mirrors``: unpacked (hi, lo) copies of the inverse roots / eigenvectors
         and their transposes.  ``exchange``: all-gather buffers or the peer-addressable arena."""

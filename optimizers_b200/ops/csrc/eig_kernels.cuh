@@ -1,7 +1,7 @@
 // Kernels of the batched eigensolver and of the QR eigenbasis refresh that are not matrix products:
 //
 //   householder_panel   Householder factorisation of one panel (up to 16 columns) of every matrix
-//                       of a batch, one CTA per matrix, the panel resident in shared memory; emits
+//                       of a batch, one CTA per matrix, the panel resident in registers (in shared memory beyond 2048 rows); emits
 //                       the compact-WY operands (V, T^T V^T, T V^T as tf32 (hi, lo) pairs) with
 //                       which the grouped tensor-core GEMM applies the block reflector to the
 //                       trailing columns and accumulates Q.  Replaces cuSOLVER geqrf / orgqr behind
