@@ -582,8 +582,6 @@ class _NewtonItem:
 
     __slots__ = (
         "block", "k", "d", "root", "power", "A", "Ar", "X", "M", "Mp", "R", "T", "pw", "err", "converged", "last_err", "iters",
-        "z",  # start scale (iterations on half pairs only)
-        "full",  # their result as a plain fp32 matrix
     )
 
 
@@ -668,7 +666,7 @@ def batched_newton_refresh(
         it = _NewtonItem()
         it.block, it.k, it.d, it.root, it.power, it.A = b, k, A.shape[0], root.numerator, root.denominator, A
         it.converged, it.last_err, it.iters = False, float("inf"), 0
-        it.Ar = it.z = it.full = None
+        it.Ar = None
         items.append(it)
     # One read for all factors: largest entries (finite?) and, for Newton, the norms of the ridged factors.
     mats = [it.A for it in items]
@@ -686,12 +684,6 @@ def batched_newton_refresh(
     # allocation and the iterates of all factors from one launch: a dozen tensors per factor, each with a fill
     # launch of its own, were half of a refresh's host time.
     errs = torch.zeros(len(items), device=device)
-    if higher is None and device.type == "cuda":  # (the stand-in of the extension on a CPU has fp32 operands)
-        for n, it in enumerate(items):
-            norm = measures[len(items) + n]
-            it.z = (it.root + 1) / (2 * norm) if norm > 0.0 else float("inf")
-            it.err = errs[n : n + 1]
-        return _newton_iterate(ext, items, errs, split, status, max_iterations, tolerance, check_every, blocks)
     sizes = [it.d for it in items for _ in range(5)]
     pairs = [(hi, lo) for _, hi, lo in ext.alloc_mat_batch(sizes, sizes, False, True, device)]
     start = []
@@ -746,11 +738,8 @@ def _newton_iterate(ext, items, errs, split, status, max_iterations, tolerance, 
     # results -> packed checkpoint state; one finiteness read
     good = [it for it in items if id(it) not in failures]
     if good:
-        if good[0].full is not None:
-            full = [it.full for it in good]
-        else:
-            pairs = [_v(it.X, it.d) for it in good]
-            full = torch._foreach_add([hi for hi, _ in pairs], [lo for _, lo in pairs])
+        pairs = [_v(it.X, it.d) for it in good]
+        full = torch._foreach_add([hi for hi, _ in pairs], [lo for _, lo in pairs])
         states, pack_specs = [], []
         for it, X in zip(good, full, strict=True):
             kf = it.block.factors
@@ -781,9 +770,6 @@ def _newton_iterate(ext, items, errs, split, status, max_iterations, tolerance, 
 
 
 def _newton_run_chunk(ext, chunk, p, errs, split, status, max_iterations, tolerance, check_every, failures, order=0) -> None:
-    if chunk[0].z is not None:
-        _newton_run_chunk_on_pairs(ext, chunk, p, errs, status, max_iterations, tolerance, check_every, failures)
-        return
     device = errs.device
     alpha = -1.0 / p
     chain = _power_chain(p)
@@ -903,94 +889,6 @@ def _newton_run_chunk(ext, chunk, p, errs, split, status, max_iterations, tolera
         _verify_and_power(ext, [it for it in chunk if id(it) not in failures], p, chain, gemm, errs, split, status, failures)
     for it in chunk:  # release iteration buffers
         it.M = it.Mp = it.pw = it.A = it.R = it.T = it.Ar = None
-
-
-def _newton_run_chunk_on_pairs(ext, chunk, p, errs, status, max_iterations, tolerance, check_every, failures) -> None:
-    """The coupled Newton iteration with its matrices as scaled fp16 pairs (twice the tf32 rate, half the operand bytes,
-    the smaller accumulation error).  Bounds of the spectra, and with them of the entries, are known beforehand:
-    M starts below (p + 1) / 2 and stays below 1 after a step, M_p below (p + 1) / p and its powers below e, and X
-    grows by at most (p + 1) / p per step, so its bound is advanced on the device along with it.  Eleven factors of 600
-    and 1024 on one B200: 9.1 -> 7.2 ms per refresh step, error of the roots against fp64 4.4e-5 -> 3.8e-5."""
-    device = errs.device
-    alpha, growth = -1.0 / p, (p + 1.0) / p
-    chain = _power_chain(p)
-    sizes = [it.d for it in chunk]
-    bound = max(8.0, p + 1.0)
-    fixed = torch.tensor([bound, 0.0], device=device)
-    x_meta = [torch.tensor([[it.z ** (1.0 / p), 0.0] for it in chunk], device=device), torch.zeros(len(chunk), 2, device=device)]
-    # full-precision copies: M (source of the affine step and of the error measure) and X (the result)
-    M_full = [[full for full, _, _ in ext.alloc_mat_batch(sizes, sizes, True, False, device)] for _ in range(2)]
-    X_full = [full for full, _, _ in ext.alloc_mat_batch(sizes, sizes, True, False, device)]
-    X, M = ([ext.alloc_pair_batch(sizes, device) for _ in range(2)] for _ in range(2))
-    Mp = ext.alloc_pair_batch(sizes, device)
-    powers = {e: ext.alloc_pair_batch(sizes, device) for e, _, _ in chain}
-    index = range(len(chunk))
-    start = [(it.A, M_full[0][n], None, None, it.z, 0.0) for n, it in enumerate(chunk)]
-    start += [(it.A, X_full[n], None, None, 0.0, it.z ** (1.0 / p)) for n, it in enumerate(chunk)]
-    ext.shift_scale_split(*ext.build_sym_table(start))
-    m_meta = fixed.repeat(len(chunk), 1)  # the conversion raises a bound it is given only if an entry exceeds it
-    ext.pair_mirrors(*ext.build_pair_table(
-        [(M_full[0][n], M[0][n], None, m_meta[n]) for n in index] + [(X_full[n], X[0][n], None, x_meta[0][n]) for n in index]
-    ))
-    for it in chunk:
-        it.A = None
-
-    def gemm(a, b, out, c=None, a_meta=fixed, d_meta=fixed):
-        # symmetric and mirrored bit for bit, see _newton_run_chunk
-        flags = ext.FLAG_MIRROR | ext.FLAG_SPLIT_OUT | ext.FLAG_FIXED_SCALE | (0 if c is not None else ext.FLAG_NO_C)
-        return (a, None, b, None, c, out, None, None, 0 if c is None else c.stride(0), out.stride(0), flags, True,
-                None, None, (a_meta, fixed, d_meta))
-
-    def build(active, cur):
-        nxt = cur ^ 1
-        affine = ext.build_mat_table([(M_full[cur][n], Mp[n], None, None, bound) for n in active])
-        stages = [[gemm(X[cur][n], Mp[n], X[nxt][n], X_full[n], x_meta[cur][n], x_meta[nxt][n]) for n in active]]
-        for k, (e, l, r) in enumerate(chain):
-            of = lambda q: Mp if q == 1 else powers[q]  # noqa: E731
-            specs = [gemm(of(l)[n], of(r)[n], powers[e][n]) for n in active]
-            if k == 0:
-                stages[0] += specs  # independent of X <- X M_p: same launch
-            else:
-                stages.append(specs)
-        top = Mp if p == 1 else powers[p]
-        stages.append([gemm(top[n], M[cur][n], M[nxt][n], M_full[nxt][n]) for n in active])
-        errors = ext.build_mat_table([(M_full[nxt][n], None, None, chunk[n].err) for n in active])
-        return affine, [ext.build_gemm_plan(s) for s in stages], errors
-
-    active, cur, iteration, tables = list(index), 0, 0, {}
-    while active:
-        if cur not in tables:
-            tables[cur] = build(active, cur)
-        affine, plans, errors = tables[cur]
-        torch.mul(x_meta[cur], growth, out=x_meta[cur ^ 1])
-        ext.affine_identity_split(*affine, alpha, 1.0 - alpha)
-        for plan in plans:
-            ext.run_gemm_plan(*plan, 1.0, 0.0, ext.HALF_PAIR_SYM, status)
-        iteration += 1
-        cur ^= 1
-        if iteration % check_every and iteration < max_iterations:
-            continue
-        errs.zero_()
-        ext.identity_error(*errors)
-        values = torch.stack([chunk[n].err[0] for n in active]).cpu().tolist()  # the only host read of the loop
-        still = []
-        for n, e in zip(active, values, strict=True):
-            it = chunk[n]
-            it.iters = iteration
-            stalled = e < 1e-3 and e > 0.9 * it.last_err
-            if e != e or e == float("inf"):
-                failures[id(it)] = ArithmeticError("coupled Newton iteration produced NaN/Inf")
-            elif e <= tolerance or stalled or iteration >= max_iterations:
-                if e > tolerance and iteration >= max_iterations:
-                    logger.warning("Newton did not converge and reached maximum number of iterations!")
-            else:
-                it.last_err = e
-                still.append(n)
-                continue
-            it.full = X_full[n]  # no later launch writes it: the factor has left the tables
-        if len(still) != len(active):
-            tables = {}
-        active = still
 
 
 def _verify_and_power(ext, items, p, chain, gemm, errs, split, status, failures) -> None:

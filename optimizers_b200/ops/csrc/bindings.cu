@@ -793,12 +793,6 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t> build_mat_table(const std::vec
       op.dst_lo = lo->data_ptr<float>();
     }
     op.err = fptr(s[3].cast<std::optional<torch::Tensor>>());
-    if (s.size() == 5) {  // half pairs of the given bound
-      op.bound = s[4].cast<float>();
-      TORCH_CHECK(op.bound > 0.f && hi.has_value() && !lo.has_value() && op.ld_dst % kBK == 0 && hi->size(1) == op.ld_dst && op.ld_dst >= op.d &&
-                      hi->size(0) >= op.d && reinterpret_cast<uintptr_t>(op.dst_hi) % 16 == 0,
-                  "half-pair destination must be padded to a multiple of ", kBK, " columns");
-    }
     for (int r = 0; r < (op.d + kMatRowsPerChunk - 1) / kMatRowsPerChunk; ++r) chunks.push_back(make_int2(static_cast<int>(i), r));
   }
   auto d_ops = upload_bytes(ops.data(), ops.size() * sizeof(MatOp), device);

@@ -1,6 +1,5 @@
 // See flat_kernels.cuh.
 #include "flat_kernels.cuh"
-#include "half_pair.cuh"
 #include "ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -67,28 +66,6 @@ __global__ void __launch_bounds__(256) affine_identity_split_kernel(const MatOp*
     const MatOp op = ops[ref.x];
     const int row0 = ref.y * kMatRowsPerChunk;
     const int rows = min(kMatRowsPerChunk, op.d - row0);
-    if (op.bound > 0.f) {  // half pairs, up to the end of the last chunk
-      const int groups = op.ld_dst >> 2;
-      const bool vec_src = (op.ld_src & 3) == 0 && (reinterpret_cast<uintptr_t>(op.src) & 15) == 0;
-      const float scale = pair_scale(op.bound);
-      for (int e = threadIdx.x; e < rows * groups; e += blockDim.x) {
-        const int i = row0 + e / groups, j = (e % groups) * 4;
-        const float* src = op.src + static_cast<long long>(i) * op.ld_src + j;
-        float x[4] = {0.f, 0.f, 0.f, 0.f};
-        if (vec_src && j + 4 <= op.d) {
-          const float4 v = *reinterpret_cast<const float4*>(src);
-          x[0] = a * v.x; x[1] = a * v.y; x[2] = a * v.z; x[3] = a * v.w;
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] = j + k < op.d ? a * src[k] : 0.f;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (i == j + k) x[k] += b;
-        store_pair4(op.dst_hi + static_cast<long long>(i) * op.ld_dst, j, x, scale);
-      }
-      continue;
-    }
     const bool vec = ((op.d | op.ld_src | op.ld_dst) & 3) == 0 &&
                      ((reinterpret_cast<uintptr_t>(op.src) | reinterpret_cast<uintptr_t>(op.dst_hi) |
                        reinterpret_cast<uintptr_t>(op.dst_lo)) & 15) == 0;

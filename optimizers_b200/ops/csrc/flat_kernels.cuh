@@ -75,8 +75,7 @@ struct MatOp {
   float* dst_hi;     // d x d, row pitch ld_dst (tf32-rounded part, or the plain result when dst_lo is null)
   float* dst_lo;     // residual part, may be null
   float* err;        // one float per matrix (identity_error)
-  int d, ld_src, ld_dst;
-  float bound;       // > 0: affine_identity_split writes dst_hi as half pairs (half_pair.cuh) of this bound, without a dst_lo
+  int d, ld_src, ld_dst, pad_;
 };
 
 constexpr int kMatRowsPerChunk = 8;

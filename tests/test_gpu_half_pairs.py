@@ -163,18 +163,3 @@ def test_plans_of_one_format_are_not_run_in_another(ext):
         ext.run_gemm_plan(*pairs, 1.0, 0.0, True, status)
     with pytest.raises(RuntimeError, match="operand format"):
         ext.run_gemm_plan(*plain, 1.0, 0.0, ext.HALF_PAIR, status)
-
-
-@pytest.mark.parametrize("sizes", [(1,), (5, 33), (128, 40, 257)])
-@pytest.mark.parametrize("bound", [8.0, 11.0])
-def test_affine_identity_on_pairs(ext, sizes, bound):
-    """a S + b I as half pairs of a given bound (the M_p of the coupled Newton iteration)."""
-    gen = torch.Generator(device="cuda").manual_seed(sum(sizes))
-    meta = torch.tensor([bound, 0.0], device="cuda")
-    mats = [torch.randn(n, n, device="cuda", generator=gen) for n in sizes]
-    outs = [torch.full((n, _pad(n)), float("nan"), device="cuda") for n in sizes]
-    ext.affine_identity_split(*ext.build_mat_table([(m, o, None, None, bound) for m, o in zip(mats, outs)]), -0.25, 1.25)
-    for m, o, n in zip(mats, outs, sizes):
-        want = -0.25 * m.double() + 1.25 * torch.eye(n, device="cuda")
-        # one fp32 rounding of the sum, then 22 bits or half a subnormal step
-        assert bool(((_value(o, meta, n) - want).abs() <= 2.0**-21 * want.abs() + 2.0**-25 / _scale(meta) + 2.0**-24).all())
