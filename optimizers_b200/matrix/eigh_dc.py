@@ -79,6 +79,7 @@ LEAF = 128  # largest problem the Jacobi kernel takes
 _MAX_ATTEMPTS = 3  # sign computations per subproblem before its root is given up
 _MAX_ROUNDS = 40  # rounds of the work list before the remaining roots are given up
 _IDEMPOTENCY_TOL = 0.05  # bound on |trace(P) - ||P||_F^2| = |sum p (1 - p)| over the eigenvalues p of P
+_ONE_BOUND = 2**30  # rows per bound of an array with one bound for all
 _SIGN_BOUND = 8.0  # of the entries of X, X^2 and W in the sign iteration (their spectra stay below 4)
 _NUDGE = 3e-5  # relative shift of the split point for a repeated sign computation
 
@@ -557,99 +558,30 @@ class NativeBackend:
             s.mean, s.mean_spread = mean, spread
 
     def sign_projector(self, subs: list[Sub]) -> None:
-        ext, dev = self.ext, self.device
-        if dev.type == "cuda":  # (the stand-in of the extension on a CPU has fp32 operands)
-            self._sign_projector_on_pairs(subs)
-            return
-        start = _mats(ext, dev, [(s.n, s.n) for s in subs], plain=False)
-        table = ext.build_sym_table(
-            [(s.A.plain, start[i].hi, start[i].lo, None, 1.0 / s.spread, -s.sigma / s.spread) for i, s in enumerate(subs)]
-        )
-        ext.shift_scale_split(*table)
-        todo, X0 = list(subs), start
-        for stage, schedule in enumerate(SIGN_STAGES):
-            projectors = self._sign_stage(todo, X0, schedule)
-            self.sign_stages_run[stage] += len(todo)
-            again, again_x = [], []
-            for s, P in zip(todo, projectors, strict=True):
-                s.extra["P"] = P
-                if stage + 1 < len(SIGN_STAGES) and s.rank >= 0 and not abs(s.idem_err) <= _IDEMPOTENCY_TOL:
-                    # not a projector yet: X = 2 P - I goes through the next stage (an elementwise pass)
-                    X = _Mat(s.n, s.n, dev)
-                    torch.add(P.hi, P.lo, out=X.plain)
-                    again.append(s)
-                    again_x.append(X)
-            if not again:
-                break
-            table = ext.build_sym_table([(X.plain, X.hi, X.lo, None, 2.0, -1.0) for X in again_x])
-            ext.shift_scale_split(*table)
-            todo, X0 = again, again_x
-
-    def _sign_stage(self, subs: list[Sub], X0: list[_Mat], schedule: tuple) -> list[_Mat]:
-        """The polynomials of ``schedule`` applied to the iterates ``X0`` (operand pairs), the last
-        one fused with P = X / 2 + I / 2; sets ``rank`` and ``idem_err`` of ``subs`` from the
-        epilogue's ||P||_F^2 and trace(P) and returns the projectors."""
-        ext, dev, F = self.ext, self.device, self.ext
-        square = [(s.n, s.n) for s in subs]
-        X = [X0, _mats(ext, dev, square, plain=False)]
-        Y = _mats(ext, dev, square)
-        W = _mats(ext, dev, square, plain=False)
-        stats = torch.zeros(len(subs), 2, device=dev)
-        idx = range(len(subs))
-        plans = []
-        for cur in (0, 1):
-            nxt = cur ^ 1
-            g1 = [self._spec(X[cur][i], X[cur][i], Y[i], c=Y[i].plain, sym=True) for i in idx]
-            # W = c Y Y + b Y + a I: beta applies to the plain copy of Y that C holds
-            g2 = [self._spec(Y[i], Y[i], W[i], c=Y[i].plain, flags=F.FLAG_ADD_DIAG, sym=True) for i in idx]
-            g3 = [self._spec(X[cur][i], W[i], X[nxt][i], sym=True) for i in idx]
-            plans.append([ext.build_gemm_plan(g) for g in (g1, g2, g3)])
-        cur = 0
-        last = len(schedule) - 1
-        for it, (a, b, c) in enumerate(schedule):
-            p1, p2, p3 = plans[cur]
-            ext.run_gemm_plan(*p1, 1.0, 0.0, True, self.status)
-            ext.run_gemm_plan(*p2, c, b, True, self.status, a)
-            if it == last:
-                # P = X W / 2 + I / 2 with ||P||_F^2 and trace(P) from the epilogue
-                final = [
-                    self._spec(X[cur][i], W[i], X[cur ^ 1][i], flags=F.FLAG_ADD_DIAG | F.FLAG_SUMSQ | F.FLAG_TRACE,
-                               sumsq=stats[i], sym=True)
-                    for i in idx
-                ]
-                self._gemm(final, 0.5, 0.0, 0.5)
-            else:
-                ext.run_gemm_plan(*p3, 1.0, 0.0, True, self.status)
-            cur ^= 1
-        for s, (fro2, trace) in zip(subs, stats.cpu().tolist(), strict=True):
-            finite = fro2 == fro2 and abs(fro2) != float("inf")
-            s.rank = int(round(fro2)) if finite else -1
-            s.idem_err = trace - fro2 if finite else float("nan")
-        return [X[cur][i] for i in idx]
-
-    def _sign_projector_on_pairs(self, subs: list[Sub]) -> None:
-        """``sign_projector`` with the iteration's matrices as scaled fp16 pairs: twice the tf32 rate and half the
+        """P = (I + sign(A - sigma I)) / 2, with the iteration's matrices as fp16 pairs: twice the tf32 rate and half the
         operand bytes, with the smaller accumulation error.  Every matrix of the iteration is a polynomial in
         X whose spectrum the schedule keeps within a few units, and no entry exceeds the spectral norm:
-        one bound serves them all.  The projector leaves as the tf32 pair its readers take."""
+        one bound serves all rows.  The projector leaves as the tf32 pair its readers take."""
         ext, dev = self.ext, self.device
-        bound = torch.tensor([_SIGN_BOUND, 0.0], device=dev)
-        sizes = [s.n for s in subs]
+        bound = torch.tensor([_SIGN_BOUND], device=dev)
 
         def start(sources, scales, todo):
-            plain = _mats(ext, dev, [(s.n, s.n) for s in todo], pair=False)
+            sizes = [s.n for s in todo]
+            plain = _mats(ext, dev, [(n, n) for n in sizes], pair=False)
             ext.shift_scale_split(*ext.build_sym_table(
                 [(src, m.plain, None, None, a, b) for src, m, (a, b) in zip(sources, plain, scales, strict=True)]
             ))
-            pairs = ext.alloc_pair_batch([s.n for s in todo], dev)
-            metas = torch.zeros(len(todo), 2, device=dev)
-            ext.pair_mirrors(*ext.build_pair_table([(m.plain, x, None, metas[i]) for i, (m, x) in enumerate(zip(plain, pairs, strict=True))]))
-            return pairs, list(metas)
+            pairs = ext.alloc_pair_batch(sizes, dev)
+            rows = torch.empty(sum(sizes), device=dev).split(sizes)
+            ext.pair_mirrors(*ext.build_pair_table(
+                [(m.plain, x, (r, None, None), None) for m, x, r in zip(plain, pairs, rows, strict=True)]
+            ))
+            return pairs, [(r, 1) for r in rows]
 
         todo = list(subs)
         X0 = start([s.A.plain for s in subs], [(1.0 / s.spread, -s.sigma / s.spread) for s in subs], subs)
         for stage, schedule in enumerate(SIGN_STAGES):
-            projectors = self._sign_stage_on_pairs(todo, *X0, schedule, bound)
+            projectors = self._sign_stage(todo, *X0, schedule, (bound, _ONE_BOUND))
             self.sign_stages_run[stage] += len(todo)
             again = []
             for s, P in zip(todo, projectors, strict=True):
@@ -662,7 +594,10 @@ class NativeBackend:
             sums = torch._foreach_add([s.extra["P"].hi for s in again], [s.extra["P"].lo for s in again])
             todo, X0 = again, start(sums, [(2.0, -1.0)] * len(again), again)
 
-    def _sign_stage_on_pairs(self, subs: list[Sub], X0: list[Tensor], metas: list[Tensor], schedule: tuple, bound: Tensor) -> list[_Mat]:
+    def _sign_stage(self, subs: list[Sub], X0: list[Tensor], rows0: list[tuple], schedule: tuple, fixed: tuple) -> list[_Mat]:
+        """The polynomials of ``schedule`` applied to the iterates ``X0`` (half pairs, with the bounds of their rows), the last
+        one fused with P = X / 2 + I / 2; sets ``rank`` and ``idem_err`` of ``subs`` from the
+        epilogue's ||P||_F^2 and trace(P) and returns the projectors."""
         ext, dev, F = self.ext, self.device, self.ext
         sizes, idx = [s.n for s in subs], range(len(subs))
         X = [X0, ext.alloc_pair_batch(sizes, dev), ext.alloc_pair_batch(sizes, dev)]  # the start (own bounds), then in turn
@@ -671,22 +606,22 @@ class NativeBackend:
         stats = torch.zeros(len(subs), 2, device=dev)
         sym = F.FLAG_MIRROR | F.FLAG_SPLIT_OUT | F.FLAG_FIXED_SCALE
 
-        def spec(a, b, a_meta, b_meta, out, c, flags):
+        def spec(a, b, a_rows, b_rows, out, c, flags):
             c_ld = 0 if c is None else c.stride(0)
             return (a, None, b, None, c, out, None, None, c_ld, out.stride(0), flags | sym | (F.FLAG_NO_C if c is None else 0), True,
-                    None, None, (a_meta, b_meta, bound))
+                    None, None, (*a_rows, *b_rows, (None, None, None, fixed[0])))
 
         plans = {}
         # W = c Y Y + b Y + a I: beta applies to the plain copy of Y that C holds
-        second = ext.build_gemm_plan([spec(Y[i], Y[i], bound, bound, W[i], Yp[i], F.FLAG_ADD_DIAG) for i in idx])
-        meta = lambda cur, i: metas[i] if cur == 0 else bound  # noqa: E731
+        second = ext.build_gemm_plan([spec(Y[i], Y[i], fixed, fixed, W[i], Yp[i], F.FLAG_ADD_DIAG) for i in idx])
+        rows = lambda cur, i: rows0[i] if cur == 0 else fixed  # noqa: E731
         cur, last = 0, len(schedule) - 1
         for it, (a, b, c) in enumerate(schedule):
             nxt = 1 if cur != 1 else 2
             if cur not in plans:
                 plans[cur] = (
-                    ext.build_gemm_plan([spec(X[cur][i], X[cur][i], meta(cur, i), meta(cur, i), Y[i], Yp[i], 0) for i in idx]),
-                    ext.build_gemm_plan([spec(X[cur][i], W[i], meta(cur, i), bound, X[nxt][i], None, 0) for i in idx]) if it != last else None,
+                    ext.build_gemm_plan([spec(X[cur][i], X[cur][i], rows(cur, i), rows(cur, i), Y[i], Yp[i], 0) for i in idx]),
+                    ext.build_gemm_plan([spec(X[cur][i], W[i], rows(cur, i), fixed, X[nxt][i], None, 0) for i in idx]) if it != last else None,
                 )
             first, third = plans[cur]
             ext.run_gemm_plan(*first, 1.0, 0.0, F.HALF_PAIR_SYM, self.status)
@@ -697,7 +632,7 @@ class NativeBackend:
                 flags = F.FLAG_MIRROR | F.FLAG_SPLIT_OUT | F.FLAG_NO_C | F.FLAG_ADD_DIAG | F.FLAG_SUMSQ | F.FLAG_TRACE
                 final = [
                     (X[cur][i], None, W[i], None, None, out[i].hi, out[i].lo, stats[i], 0, out[i].hi.stride(0), flags, True,
-                     None, None, (meta(cur, i), bound, None))
+                     None, None, (*rows(cur, i), *fixed, None))
                     for i in idx
                 ]
                 ext.run_gemm_plan(*ext.build_gemm_plan(final), 0.5, 0.0, F.HALF_PAIR_SYM, self.status, 0.5)

@@ -33,7 +33,7 @@ groups of HSDP and hybrid shard) gathers the search directions with NCCL or, wit
 from __future__ import annotations
 
 import logging
-from typing import Any
+from typing import Any, NamedTuple
 
 import torch
 from torch import Tensor
@@ -76,10 +76,13 @@ def _pad4(n: int) -> int:
     return (n + 3) // 4 * 4
 
 
-# Step scratch of one block: two norms, then the (bound, squared row norm) meta data of its half-pair operands.
-# The first three slots are read by the kernels under these offsets (block_kernels.cuh, kMeta*).
-_META_GRAD, _META_FILTERED, _META_SCALED, _META_T, _META_T2, _META_U, _META_U2 = range(0, 14, 2)
-_META_SIZE = 14
+class _Rows(NamedTuple):
+    """Bounds of the rows of a half-pair operand array, on the device: the scale of a row follows from its bound."""
+
+    bound: Tensor  # of |entries|, one per row
+    top: Tensor | None = None  # the largest of them (chained products)
+    l1: Tensor | None = None  # 1-norms of the rows and the largest (inverse roots and eigenbases)
+    l1_top: Tensor | None = None
 
 
 # Configurations whose 2-D blocks may carry a factor on one dim only (the other switched off by an
@@ -219,6 +222,7 @@ class _Block:
         "dims3", "view2d", "y_hi", "y_lo", "zt_hi", "zt_lo", "aux_g_hi", "aux_g_lo", "aux_gt_hi", "aux_gt_lo", "d1_hi", "d1_lo", "d2_hi", "d2_lo",
         "e1_hi", "e1_lo", "e2_hi", "e2_lo",  # second set of chain intermediates (eigenvalue-corrected order-3: two chains per stage)
         "sel",  # per dim of the block: has a Kronecker factor (inverse_exponent_override 0 switches a dim off)
+        "rows",  # half pairs: operand array -> _Rows
         "eig_hints",  # factor index -> eigenvalues found at the previous refresh (host tensor; steers the eigensolver)
     )
 
@@ -235,8 +239,8 @@ class NativeGroupEngine:
         self._dist = rec[DISTRIBUTOR]
         self._device = group[PARAMS][0].device
         self._plist = rec[SHAMPOO_PRECONDITIONER_LIST]
-        # Operand format of the step's products at gemm_mode="tf32x3": scaled fp16 pairs (three products at
-        # twice the tf32 rate, half the operand bytes, no larger error) wherever the layouts allow it, tf32
+        # Operand format of the step's products at gemm_mode="tf32x3": fp16 pairs with a scale per row (three
+        # products at twice the tf32 rate, half the operand bytes) wherever the layouts allow it, tf32
         # (hi, lo) pairs of fp32 arrays elsewhere.  ``_split`` is the latter; the refreshes use it in both cases.
         self._refresh_split = cfg.gemm_mode == "tf32x3"
         self._half = self._refresh_split and self._half_pairs_cover(group, cfg)
@@ -325,13 +329,12 @@ class NativeGroupEngine:
     # ------------------------------------------------------------------------------------------
     def _half_pairs_cover(self, group: dict[str, Any], cfg: NativeRuntimeConfig) -> bool:
         """Half pairs interleave 32 elements along K, which an order-3 block's re-viewed unfoldings keep
-        only if its first two dims are multiples of 32.  Their scale takes a pass over the gradient before
+        only if its first two dims are multiples of 32.  Their scales take a pass over the gradient before
         the prologue, which a gradient reduced from the peers' memory does not have; the transposing copy
-        of blocks preconditioned on the rows only moves fp32 arrays.  The stand-in of the extension on a CPU
-        has fp32 operands.  Where pairs do apply they win at every size: a step over an 8192 x 8192 weight
-        takes 2.96 ms with them and 4.93 ms with tf32 pairs, one over 1000 x 1337 weights 0.19 and 0.23 ms."""
-        if self._device.type != "cuda":
-            return False
+        of blocks preconditioned on the rows only moves fp32 arrays.  Pairs keep 22 bits of an entry down to 2^-28 of its row's bound and 2^-50 of the bound
+        below (half_pair.cuh), tf32 pairs 22 bits of any entry.  A step over an 8192 x 8192 weight takes 3.1 ms with pairs
+        and 4.9 ms with tf32 pairs, one over weights of 1000 x 1337 and below 0.19 and 0.23 ms, one over a 784-512-10
+        perceptron, which the host bounds, the same with both."""
         if type(group[DISTRIBUTED_CONFIG]) is DDPDistributedConfig and cfg.comm_path == "p2p" and cfg.fuse_gradient_reduction:
             return False
         selectors = self._plist._local_preconditioned_dims_selector_list
@@ -359,12 +362,12 @@ class NativeGroupEngine:
         moms = rec.get(MOMENTUM_BUFFER_LIST)
         zs = rec.get(WEIGHT_BUFFER_LIST)
         vs = self._glist._local_preconditioner_list if self._graft_kind == _GRAFT_ADAGRAD else None
-        # Zeroed by one fill at the start of a step: the norms, and the meta data of the half-pair operands.
         count = max(len(dist.local_blocked_params), 1)
-        self._step_scratch = torch.zeros(count * (2 + (_META_SIZE if self._half else 0)), dtype=torch.float32, device=dev)
+        # Zeroed by one fill at the start of a step: the norms, and the measured bounds of the half-pair operands' rows.
+        sizes = [self._measured_rows(view) if self._half else {} for view in dist.local_blocked_params]
+        cursor = (2 * count + 31) // 32 * 32
+        self._step_scratch = torch.zeros(cursor + sum(sum(s.values()) for s in sizes), dtype=torch.float32, device=dev)
         self._norms = self._step_scratch[: 2 * count].view(count, 2)
-        self._meta = self._step_scratch[2 * count :].view(count, _META_SIZE) if self._half else None
-        self._root_meta = torch.zeros(count, 3, 2, dtype=torch.float32, device=dev) if self._half else None
 
         pool = _ZeroPool(dev)
         zeros = pool.zeros
@@ -379,6 +382,11 @@ class NativeGroupEngine:
             b.grad_slot = local_owner[i]
             b.grad_offset = (view.data_ptr() - self._local_params[b.grad_slot].data_ptr()) // 4
             b.order = view.dim()
+            b.rows = {}
+            if self._half:
+                measured = self._step_scratch[cursor : cursor + sum(sizes[i].values())].split(list(sizes[i].values()))
+                cursor += sum(sizes[i].values())
+                self._name_rows(b, dict(zip(sizes[i], measured, strict=True)))
             b.dims3 = None
             b.view2d = view
             if view.dim() == 1:
@@ -442,6 +450,34 @@ class NativeGroupEngine:
                 b.t2_lo = zeros(b.n, b.m_pad) if two_d and self._split else None
             blocks.append(b)
         self._blocks = blocks
+
+    def _measured_rows(self, view: Tensor) -> dict[str, int]:
+        """Sizes of a block's measured bounds: a number per row of each operand array the pointwise kernels write, in whole
+        chunks of 32."""
+        if view.dim() == 3:
+            a, bb, c = view.shape
+            m, aux, n = a * bb, {"aux_g": a, "aux_gt": bb}, c  # the mode-b unfolding has one row for c rows of aux_gt
+        else:
+            m, n = (1, view.shape[0]) if view.dim() == 1 else view.shape
+            aux = {}
+        scaled = {"s": m, "s_cols": n} if self._soap else {}
+        sizes = {"tops": 5, "g": m, "gt": n, "f": m, "f_cols": n, **scaled, **aux}
+        return {name: (size + 31) // 32 * 32 for name, size in sizes.items()}
+
+    def _name_rows(self, b: _Block, measured: dict[str, Tensor]) -> None:
+        """``b.rows``: the measured bounds (``measured``, zero between steps; f_cols and s_cols are of columns), those of chained
+        products (t, t2: of the filtered gradient; u, u2: of the gradient; w: of the scaled direction) and of the mirrors (root<k>; qt<k>: of
+        the transposed eigenbases)."""
+        tops = dict(zip(("t", "t2", "u", "u2", "w"), measured.pop("tops")[:5].split(1), strict=True))
+        b.rows.update((name, _Rows(bound)) for name, bound in measured.items())
+        shape = b.param_view.shape
+        for name, top in tops.items():
+            b.rows[name] = _Rows(torch.zeros(max(shape), dtype=torch.float32, device=self._device), top)
+        dims = [d for d, on in zip(shape, b.sel, strict=True) if on]
+        for name in ("root", "qt") if self._soap else ("root",):
+            for k, d in enumerate(dims):
+                flat = torch.zeros(2 * d + 1, dtype=torch.float32, device=self._device)
+                b.rows[f"{name}{k}"] = _Rows(flat[1 : d + 1], None, flat[d + 1 :], flat[:1])
 
     def _alloc_order3(self, b: _Block, zeros) -> None:
         """Operand buffers of an order-3 block (a, b, c).  Mode unfoldings, all K-major:
@@ -562,7 +598,7 @@ class NativeGroupEngine:
                     b.g_hi, b.g_lo, b.gt_hi, b.gt_lo, b.f_hi, b.f_lo, b.p, self._norms[b.index], self._send_ptr(b),
                     self._slot_offset(b), b.ev, 0 if (self._soap or any(b.sel)) else 2,
                 )
-                + ((self._meta[b.index],) if self._half else ())
+                + self._row_spec(b, "g", "gt", 1, "f", "f_cols" if b.order > 1 else None, "s", "s_cols" if b.order > 1 else None)
             )
         for b in blocks:
             if b.dims3 is None:
@@ -572,7 +608,7 @@ class NativeGroupEngine:
             specs.append(
                 (b.param_view.view(a, bb * c), b.grad_offset, b.grad_slot, a, bb * c, bb * c, a)
                 + (None,) * 4 + (b.aux_g_hi, b.aux_g_lo, b.aux_gt_hi, b.aux_gt_lo) + (None,) * 4 + (0, 0, None, 1)
-                + ((self._meta[b.index],) if self._half else ())
+                + self._row_spec(b, "aux_g", "aux_gt", c, None, None, None, None)
             )
         self._table = ext.build_block_table(specs)
         if self._soap:
@@ -589,8 +625,10 @@ class NativeGroupEngine:
             return
 
         op = self._operand
-        meta = self._with_meta
+        rows = self._with_rows
         syrk, gemm0, gemm1, gemm2, kl = [], [], [], [], []
+        chain_rows, kl_rows = [], []  # bounds of chained products
+        from_columns = self._from_columns
         f_transposes = []  # (F hi|lo -> T^T hi|lo) of the blocks preconditioned on the rows only
         pack_flag = F.FLAG_PACKED_C if self._packing else 0
         sp = self._split
@@ -609,15 +647,15 @@ class NativeGroupEngine:
                 xa = (b.aux_g_hi, lo(b.aux_g_lo))
                 xb = (b.aux_gt_hi.view(bb, c * a), lo(b.aux_gt_lo.view(bb, c * a) if sp else None))
                 xc = (b.gt_hi, lo(b.gt_lo))
-                for (x_hi, x_lo), factor, d in ((xa, fm[0], a), (xb, fm[1], bb), (xc, fm[2], c)):
-                    syrk.append(meta(b, (x_hi, x_lo, x_hi, x_lo, factor, None, None, None, d, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                for (x_hi, x_lo), factor, d, name in ((xa, fm[0], a, "aux_g"), (xb, fm[1], bb, "aux_gt"), (xc, fm[2], c, "gt")):
+                    syrk.append(rows(b, (x_hi, x_lo, x_hi, x_lo, factor, None, None, None, d, 0, pack_flag, self._packing), name, name))
                 inv = [(op(b.inv_hi[k], d, d), op(b.inv_lo[k], d, d) if sp else None) for k, d in enumerate(b.dims3)]
                 f = (op(b.f_hi, a * bb, c), op(b.f_lo, a * bb, c) if sp else None)
-                gemm0.append(meta(b, chained(*inv[2], *f, b.d1_hi, b.d1_lo), "root2", _META_FILTERED, _META_T))
+                gemm0.append(rows(b, chained(*inv[2], *f, b.d1_hi, b.d1_lo), "root2", "f", from_columns(chain_rows, b, b.inv_hi[2], "root2", "f_cols", "t")))
                 d1 = (b.d1_hi.view(c * a, bb), lo(b.d1_lo.view(c * a, bb) if sp else None))
-                gemm1.append(meta(b, chained(*inv[1], *d1, b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
+                gemm1.append(rows(b, chained(*inv[1], *d1, b.d2_hi, b.d2_lo), "root1", "t", self._second_of_three(b, "root1"), a))
                 d2 = (b.d2_hi.view(bb * c, a), lo(b.d2_lo.view(bb * c, a) if sp else None))
-                gemm2.append(meta(b, (*inv[0], *d2, b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", _META_T2))
+                gemm2.append(rows(b, (*inv[0], *d2, b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", "t2", div=c))
                 continue
             two_d = b.order == 2
             left, right = two_d and b.sel[0], b.sel[-1]
@@ -633,18 +671,18 @@ class NativeGroupEngine:
                 a_hi, a_lo = op(b.g_hi, b.m, b.n), (op(b.g_lo, b.m, b.n) if sp else None)
                 ri = (op(b.inv_hi[1], b.n, b.n), op(b.inv_lo[1], b.n, b.n) if sp else None)
                 li = (op(b.inv_hi[0], b.m, b.m), op(b.inv_lo[0], b.m, b.m) if sp else None)
-                kl.append(meta(b, chained(a_hi, a_lo, *ri, b.y_hi, b.y_lo), _META_GRAD, "root1", _META_U))
-                kl.append(meta(b, chained(t_hi, t_lo, *li, b.zt_hi, b.zt_lo), _META_GRAD, "root0", _META_U2))
+                kl.append(rows(b, chained(a_hi, a_lo, *ri, b.y_hi, b.y_lo), "g", "root1", self._kl_rows(kl_rows, b, 1, "g", "gt", "t", "u")))
+                kl.append(rows(b, chained(t_hi, t_lo, *li, b.zt_hi, b.zt_lo), "gt", "root0", self._kl_rows(kl_rows, b, 0, "gt", "g", "t2", "u2")))
                 y = (op(b.y_hi, b.m, b.n), op(b.y_lo, b.m, b.n) if sp else None)
                 zt = (op(b.zt_hi, b.n, b.m), op(b.zt_lo, b.n, b.m) if sp else None)
-                syrk.append(meta(b, (*y, *y, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_U, _META_U))
-                syrk.append(meta(b, (*zt, *zt, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_U2, _META_U2))
+                syrk.append(rows(b, (*y, *y, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), "u", "u"))
+                syrk.append(rows(b, (*zt, *zt, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), "u2", "u2"))
             else:
                 if left:
                     a_hi, a_lo = op(b.g_hi, b.m, b.n), (op(b.g_lo, b.m, b.n) if self._split else None)
-                    syrk.append(meta(b, (a_hi, a_lo, a_hi, a_lo, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                    syrk.append(rows(b, (a_hi, a_lo, a_hi, a_lo, fm[0], None, None, None, b.m, 0, pack_flag, self._packing), "g", "g"))
                 if right:
-                    syrk.append(meta(b, (t_hi, t_lo, t_hi, t_lo, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                    syrk.append(rows(b, (t_hi, t_lo, t_hi, t_lo, fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), "gt", "gt"))
 
             f_hi, f_lo = op(b.f_hi, b.m, b.n), (op(b.f_lo, b.m, b.n) if self._split else None)
             sumsq = self._norms[b.index, 1:2]
@@ -659,13 +697,14 @@ class NativeGroupEngine:
             elif left:
                 r_hi, r_lo = op(b.inv_hi[1], b.n, b.n), (op(b.inv_lo[1], b.n, b.n) if self._split else None)
                 l_hi, l_lo = op(b.inv_hi[0], b.m, b.m), (op(b.inv_lo[0], b.m, b.m) if self._split else None)
-                gemm1.append(meta(b, chained(r_hi, r_lo, f_hi, f_lo, b.tt_hi, b.tt_lo), "root1", _META_FILTERED, _META_T))
+                gemm1.append(rows(b, chained(r_hi, r_lo, f_hi, f_lo, b.tt_hi, b.tt_lo), "root1", "f", from_columns(chain_rows, b, b.inv_hi[1], "root1", "f_cols", "t")))
                 tt_hi, tt_lo = op(b.tt_hi, b.n, b.m), (op(b.tt_lo, b.n, b.m) if self._split else None)
-                gemm2.append(meta(b, (l_hi, l_lo, tt_hi, tt_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", _META_T))
+                gemm2.append(rows(b, (l_hi, l_lo, tt_hi, tt_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", "t"))
             else:  # columns only: a 1-D block, or a 2-D block whose rows are not preconditioned
                 r_hi, r_lo = op(b.inv_hi[-1], b.n, b.n), (op(b.inv_lo[-1], b.n, b.n) if self._split else None)
                 root = f"root{len(b.inv_hi) - 1}"
-                gemm2.append(meta(b, (f_hi, f_lo, r_hi, r_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), _META_FILTERED, root))
+                gemm2.append(rows(b, (f_hi, f_lo, r_hi, r_lo, b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "f", root))
+        self._chain_rows, self._kl_rows_table = self._row_bound_table(chain_rows), self._row_bound_table(kl_rows)
         self._f_transpose_table = ext.build_transpose_table(f_transposes) if f_transposes else None
         # the pushing plan pairs one final product with every block (see the rule at _gemm_push)
         assert not self._gemm_push or len(gemm2) == len(blocks)
@@ -687,16 +726,48 @@ class NativeGroupEngine:
         """The K extent of an operand array the products read (half pairs: whole chunks, zero padded)."""
         return t[:, :k] if t.shape[1] != k and not self._half else t
 
-    def _with_meta(self, b: _Block, spec: tuple, a_slot: int | str, b_slot: int | str, d_slot: int | None = None) -> tuple:
-        """``spec`` with the meta data of its half-pair operands and split output: slots of the block's step
-        scratch, or ``"root<k>"`` for the mirror of its k-th inverse root (or eigenbasis, or its transpose)."""
+    def _row_spec(self, b: _Block, g: str, gt: str, col_div: int, *others: str | None) -> tuple:
+        if not self._half:
+            return ()
+        of = lambda name: b.rows[name].bound if name in b.rows else None  # noqa: E731
+        return ((of(g), of(gt), col_div, *map(of, others)),)
+
+    def _with_rows(self, b: _Block, spec: tuple, left: str, right: str, out: tuple | None = None, div: int = 1) -> tuple:
+        """``spec`` with the bounds (names in ``b.rows``) of the rows of its half-pair operands and, if it is chained, of its
+        result: ``out`` is what ``_from_columns`` or ``_from_norms`` gave.  ``div``: view rows of the right operand per row it
+        was written with."""
         if not self._half:
             return spec
+        return (*spec, None, None, (b.rows[left].bound, 1, b.rows[right].bound, div, out))
 
-        def of(slot):
-            return self._root_meta[b.index, int(slot[4:])] if isinstance(slot, str) else self._meta[b.index, slot : slot + 2]
+    def _from_columns(self, table: list, b: _Block, mirror: Tensor, rows: str, columns: str, out: str) -> tuple | None:
+        """Bounds of the rows of ``mirror X^T``, from the mirror and the largest entries of the columns of X: adds the launch
+        that finds them to ``table``."""
+        if not self._half:
+            return None
+        d = b.rows[out]
+        table.append((mirror, b.rows[rows].bound, b.rows[columns].bound, d.bound, d.top))
+        return (None, None, None, d.bound)
 
-        return (*spec, None, None, (of(a_slot), of(b_slot), None if d_slot is None else of(d_slot)))
+    def _from_norms(self, b: _Block, left: Tensor, right: Tensor, out: str, cap: Tensor | None = None) -> tuple | None:
+        """Bounds left[i] right[0] (at most ``cap[0]``) of the rows of a result, written by the product's epilogue."""
+        return (left, right, cap, b.rows[out].bound) if self._half else None
+
+    def _second_of_three(self, b: _Block, mirror: str, first: str = "t", out: str = "t2") -> tuple | None:
+        return self._from_norms(b, b.rows[mirror].l1, b.rows[first].top, out) if self._half else None
+
+    def _kl_rows(self, table: list, b: _Block, k: int, rows: str, columns: str, scratch: str, out: str) -> tuple | None:
+        """Bounds of the rows of ``X S`` with S the k-th root: the row's largest entry times the largest 1-norm of a row of S, at
+        most what the columns of X give for the whole result (a row of S may be large where X has next to nothing)."""
+        if not self._half:
+            return None
+        self._from_columns(table, b, b.inv_hi[k], f"root{k}", columns, scratch)
+        d = b.rows[out]
+        table[-1] = (*table[-1][:4], d.top)
+        return self._from_norms(b, b.rows[rows].bound, b.rows[f"root{k}"].l1_top, out, d.top)
+
+    def _row_bound_table(self, specs: list) -> tuple | None:
+        return self._ext.build_row_bound_table(specs) if specs else None
 
     def _build_soap_plans(self, blocks: list[_Block]) -> None:
         """GEMM plans of the eigenvalue-corrected step.  With Qt the transposed eigenvector
@@ -710,7 +781,8 @@ class NativeGroupEngine:
         ext, split = self._ext, self._split
         F = ext
 
-        meta = self._with_meta
+        rows, from_columns = self._with_rows, self._from_columns
+        first_rows, back_rows = [], []  # bounds of chained products
 
         def pair(hi: Tensor, lo: Tensor | None, k: int) -> tuple[Tensor, Tensor | None]:
             return self._operand(hi, 0, k), (lo[:, :k] if lo is not None else None)
@@ -738,8 +810,8 @@ class NativeGroupEngine:
                 xa = (b.aux_g_hi, lo(b.aux_g_lo))
                 xb = (b.aux_gt_hi.view(bb, c * a), lo(b.aux_gt_lo.view(bb, c * a) if split else None))
                 xc = (b.gt_hi, lo(b.gt_lo))
-                for x, factor, d in ((xa, fm[0], a), (xb, fm[1], bb), (xc, fm[2], c)):
-                    syrk.append(meta(b, (*_ab(x, x), factor, None, None, None, d, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                for x, factor, d, name in ((xa, fm[0], a, "aux_g"), (xb, fm[1], bb, "aux_gt"), (xc, fm[2], c, "gt")):
+                    syrk.append(rows(b, (*_ab(x, x), factor, None, None, None, d, 0, pack_flag, self._packing), name, name))
                 q = [pair(b.inv_hi[k], b.inv_lo[k], d) for k, d in enumerate(b.dims3)]
                 qt = [pair(b.qt_hi[k], b.qt_lo[k], d) for k, d in enumerate(b.dims3)]
                 g3, f3 = pair(b.g_hi, b.g_lo, c), pair(b.f_hi, b.f_lo, c)
@@ -747,16 +819,16 @@ class NativeGroupEngine:
                 def as_rows(hi, lo_, rows, cols):
                     return (hi.view(rows, cols), lo_.view(rows, cols) if lo_ is not None else None)
 
-                st_a0.append(meta(b, chained(qt[2], g3, b.e1_hi, b.e1_lo), "root2", _META_GRAD, _META_U))
-                st_a0.append(meta(b, chained(qt[2], f3, b.d1_hi, b.d1_lo), "root2", _META_FILTERED, _META_T))
-                st_a.append(meta(b, chained(qt[1], as_rows(b.e1_hi, b.e1_lo, c * a, bb), b.e2_hi, b.e2_lo), "root1", _META_U, _META_U2))
-                st_a.append(meta(b, chained(qt[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
+                st_a0.append(rows(b, chained(qt[2], g3, b.e1_hi, b.e1_lo), "qt2", "g", from_columns(first_rows, b, b.qt_hi[2], "qt2", "gt", "u")))
+                st_a0.append(rows(b, chained(qt[2], f3, b.d1_hi, b.d1_lo), "qt2", "f", from_columns(first_rows, b, b.qt_hi[2], "qt2", "f_cols", "t")))
+                st_a.append(rows(b, chained(qt[1], as_rows(b.e1_hi, b.e1_lo, c * a, bb), b.e2_hi, b.e2_lo), "qt1", "u", self._second_of_three(b, "qt1", "u", "u2"), a))
+                st_a.append(rows(b, chained(qt[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "qt1", "t", self._second_of_three(b, "qt1"), a))
                 ev = b.ev.view(a, bb * c)
-                st_v.append(meta(b, (*_ab(qt[0], as_rows(b.e2_hi, b.e2_lo, bb * c, a)), ev, None, None, None, bb * c, 0, F.FLAG_SQUARE_ACC, False), "root0", _META_U2))
-                st_f.append(meta(b, (*_ab(qt[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, None, bb * c, 0, 0, False), "root0", _META_T2))
-                st_u0.append(meta(b, chained(q[2], f3, b.d1_hi, b.d1_lo), "root2", _META_SCALED, _META_T))
-                st_u1.append(meta(b, chained(q[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "root1", _META_T, _META_T2))
-                st_u2.append(meta(b, (*_ab(q[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", _META_T2))
+                st_v.append(rows(b, (*_ab(qt[0], as_rows(b.e2_hi, b.e2_lo, bb * c, a)), ev, None, None, None, bb * c, 0, F.FLAG_SQUARE_ACC, False), "qt0", "u2", div=c))
+                st_f.append(rows(b, (*_ab(qt[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, None, bb * c, 0, 0, False), "qt0", "t2", div=c))
+                st_u0.append(rows(b, chained(q[2], f3, b.d1_hi, b.d1_lo), "root2", "s", from_columns(back_rows, b, b.inv_hi[2], "root2", "s_cols", "w")))
+                st_u1.append(rows(b, chained(q[1], as_rows(b.d1_hi, b.d1_lo, c * a, bb), b.d2_hi, b.d2_lo), "root1", "w", self._second_of_three(b, "root1", "w"), a))
+                st_u2.append(rows(b, (*_ab(q[0], as_rows(b.d2_hi, b.d2_lo, bb * c, a)), b.p, None, None, self._norms[b.index, 1:2], bb * c, 0, F.FLAG_SUMSQ, False), "root0", "t2", div=c))
                 continue
             two_d = b.order == 2
             g = pair(b.g_hi, b.g_lo, b.n)
@@ -764,25 +836,26 @@ class NativeGroupEngine:
             f = pair(b.f_hi, b.f_lo, b.n)
             sumsq = self._norms[b.index, 1:2]
             if two_d:
-                syrk.append(meta(b, (*_ab(g, g), fm[0], None, None, None, b.m, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
-            syrk.append(meta(b, (*_ab(gt, gt), fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), _META_GRAD, _META_GRAD))
+                syrk.append(rows(b, (*_ab(g, g), fm[0], None, None, None, b.m, 0, pack_flag, self._packing), "g", "g"))
+            syrk.append(rows(b, (*_ab(gt, gt), fm[-1], None, None, None, b.n, 0, pack_flag, self._packing), "gt", "gt"))
             r = 1 if two_d else 0
             qr, qrt = pair(b.inv_hi[r], b.inv_lo[r], b.n), pair(b.qt_hi[r], b.qt_lo[r], b.n)
             if two_d:
                 ql, qlt = pair(b.inv_hi[0], b.inv_lo[0], b.m), pair(b.qt_hi[0], b.qt_lo[0], b.m)
                 t2, tt = pair(b.t2_hi, b.t2_lo, b.m), pair(b.tt_hi, b.tt_lo, b.m)
-                st_a.append(meta(b, chained(qrt, g, b.t2_hi, b.t2_lo), "root1", _META_GRAD, _META_U))
-                st_a.append(meta(b, chained(qrt, f, b.tt_hi, b.tt_lo), "root1", _META_FILTERED, _META_T))
-                st_v.append(meta(b, (*_ab(qlt, t2), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), "root0", _META_U))
-                st_f.append(meta(b, (*_ab(qlt, tt), b.p, None, None, None, b.n, 0, 0, False), "root0", _META_T))
-                st_u1.append(meta(b, chained(qr, f, b.tt_hi, b.tt_lo), "root1", _META_SCALED, _META_T))
-                st_u2.append(meta(b, (*_ab(ql, tt), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", _META_T))
+                st_a.append(rows(b, chained(qrt, g, b.t2_hi, b.t2_lo), "qt1", "g", from_columns(first_rows, b, b.qt_hi[1], "qt1", "gt", "u")))
+                st_a.append(rows(b, chained(qrt, f, b.tt_hi, b.tt_lo), "qt1", "f", from_columns(first_rows, b, b.qt_hi[1], "qt1", "f_cols", "t")))
+                st_v.append(rows(b, (*_ab(qlt, t2), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), "qt0", "u"))
+                st_f.append(rows(b, (*_ab(qlt, tt), b.p, None, None, None, b.n, 0, 0, False), "qt0", "t"))
+                st_u1.append(rows(b, chained(qr, f, b.tt_hi, b.tt_lo), "root1", "s", from_columns(back_rows, b, b.inv_hi[1], "root1", "s_cols", "w")))
+                st_u2.append(rows(b, (*_ab(ql, tt), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "root0", "w"))
             else:
-                st_v.append(meta(b, (*_ab(g, qrt), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), _META_GRAD, "root0"))
-                st_f.append(meta(b, (*_ab(f, qrt), b.p, None, None, None, b.n, 0, 0, False), _META_FILTERED, "root0"))
-                st_u2.append(meta(b, (*_ab(f, qr), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), _META_SCALED, "root0"))
+                st_v.append(rows(b, (*_ab(g, qrt), b.ev, None, None, None, b.n, 0, F.FLAG_SQUARE_ACC, False), "g", "qt0"))
+                st_f.append(rows(b, (*_ab(f, qrt), b.p, None, None, None, b.n, 0, 0, False), "f", "qt0"))
+                st_u2.append(rows(b, (*_ab(f, qr), b.p, None, None, sumsq, b.n, 0, F.FLAG_SUMSQ, False), "s", "root0"))
         self._syrk_plan = ext.build_gemm_plan(syrk)
         mk = lambda specs: ext.build_gemm_plan(specs) if specs else None  # noqa: E731
+        self._first_rows, self._back_rows = self._row_bound_table(first_rows), self._row_bound_table(back_rows)
         self._soap_plans = {
             "a0": mk(st_a0), "a": mk(st_a), "v": mk(st_v), "f": mk(st_f), "u0": mk(st_u0), "u1": mk(st_u1), "u2": mk(st_u2),
         }
@@ -861,12 +934,18 @@ class NativeGroupEngine:
         """Measures the fp32 matrices that stand in the mirrors ``(block, k)`` for their scale and turns them into
         half pairs in place; eigenbases also into their transposes."""
         ext = self._ext
-        metas = [self._root_meta[b.index, k] for b, k in fresh]
-        torch._foreach_zero_(metas)
-        ext.pair_mirrors(*ext.build_pair_table([
-            (b.inv_hi[k][:, : b.inv_hi[k].shape[0]], b.inv_hi[k], b.qt_hi[k] if self._soap else None, m)
-            for (b, k), m in zip(fresh, metas, strict=True)
-        ]))
+        specs = []
+        for b, k in fresh:
+            d = b.inv_hi[k].shape[0]
+            own = b.rows[f"root{k}"]
+            spec = (b.inv_hi[k][:, :d], b.inv_hi[k], (own.bound, own.l1, own.l1_top))
+            if self._soap:
+                other = b.rows[f"qt{k}"]
+                specs.append((*spec, b.qt_hi[k], (other.bound, other.l1, other.l1_top)))
+            else:
+                specs.append((*spec, None))
+        torch._foreach_zero_([bounds[2] for spec in specs for bounds in spec[2::2] if bounds is not None])
+        ext.pair_mirrors(*ext.build_pair_table(specs))
 
     # ------------------------------------------------------------------------------------------
     # Hooks called by the optimizer
@@ -1104,6 +1183,7 @@ class NativeGroupEngine:
         launches += 3 if self._half else 2
         self._mark("grad_prologue")
         if not self._soap and self._kl_plan is not None:
+            launches += self._run_row_bounds(self._kl_rows_table)
             ext.run_gemm_plan(*self._kl_plan, 1.0, 0.0, self._form, self._status)
             launches += 1
         if self._syrk_plan is not None:
@@ -1123,6 +1203,7 @@ class NativeGroupEngine:
         if self._soap:
             launches += self._soap_step(plist, graft_only)
         elif not graft_only:
+            launches += self._run_row_bounds(self._chain_rows)  # after a refresh: they follow the new roots
             if self._gemm0_plan is not None:
                 ext.run_gemm_plan(*self._gemm0_plan, 1.0, 0.0, self._form, self._status)
                 launches += 1
@@ -1162,13 +1243,19 @@ class NativeGroupEngine:
         self.launches_per_step = launches
         self._finish_update()
 
+    def _run_row_bounds(self, table: tuple | None) -> int:
+        if table is None:
+            return 0
+        self._ext.row_bounds(table)
+        return 1
+
     def _soap_step(self, plist: Any, graft_only: bool) -> int:
         """Second-moment update in the eigenbasis (every step) and, unless only the grafting
         direction is needed, project -> scale -> unproject of the filtered gradient (whose projection
         runs in the first stages either way: a step that only takes the grafting direction leaves it unread)."""
         ext, plans, split = self._ext, self._soap_plans, self._form
         run = lambda key, alpha=1.0, beta=0.0: ext.run_gemm_plan(*plans[key], alpha, beta, split, self._status)  # noqa: E731
-        launches = 0
+        launches = self._run_row_bounds(self._first_rows)
         for stage in ("a0", "a"):  # first stages of the projections: order-3 blocks only, then 2-D and order-3
             if plans[stage] is not None:
                 run(stage)
@@ -1180,6 +1267,7 @@ class NativeGroupEngine:
         run("f")
         for (blocks_t, tiles_t, n_tiles), root in self._eig_tables:
             ext.eig_scale(blocks_t, tiles_t, n_tiles, float(plist._bias_correction2), 1.0 / root, plist._epsilon, split)
+        launches += self._run_row_bounds(self._back_rows)
         for stage in ("u0", "u1"):
             if plans[stage] is not None:
                 run(stage)

@@ -174,9 +174,14 @@ class PlanBuilder {
     float* d_hi = nullptr;
     float* d_lo = nullptr;
     float* sumsq = nullptr;
-    const float* a_meta = nullptr;  // half pairs: PairMeta of both operands and of the split output
-    const float* b_meta = nullptr;
-    float* d_meta = nullptr;
+    // half pairs: see GemmProblem
+    const float* a_bound = nullptr;
+    const float* b_bound = nullptr;
+    int a_div = 1, b_div = 1;
+    const float* d_left = nullptr;
+    const float* d_right = nullptr;
+    const float* d_cap = nullptr;
+    float* d_bound = nullptr;
     int M = 0, N = 0, K = 0, ldc = 0, ldd = 0, flags = 0;
     long long push_offset = 0;
     bool upper_tiles_only = false;
@@ -220,16 +225,22 @@ class PlanBuilder {
                   "mirrored output needs a square, unpacked upper-tile problem");
     }
     if (!(p.flags & kFlagNoC)) TORCH_CHECK(p.c != nullptr, "C is required unless kFlagNoC is set");
-    p.a_meta = q.a_meta;
-    p.b_meta = q.b_meta;
-    p.d_meta = q.d_meta;
-    const bool half = p.a_meta != nullptr;
+    p.a_bound = q.a_bound;
+    p.b_bound = q.b_bound;
+    p.a_div = q.a_div;
+    p.b_div = q.b_div;
+    p.d_left = q.d_left;
+    p.d_right = q.d_right;
+    p.d_cap = q.d_cap;
+    p.d_bound = q.d_bound;
+    const bool half = p.a_bound != nullptr;
     const bool half_sym = half && (p.flags & (kFlagMirror | kFlagFixedScale)) != 0;
     TORCH_CHECK(problems_.empty() || (half == half_ && half_sym == half_sym_), "a plan holds one operand format");
     half_ = half;
     half_sym_ = half_sym;
     if (half) {
-      TORCH_CHECK(p.b_meta != nullptr, "both operands of a half-pair product need their meta data");
+      TORCH_CHECK(p.b_bound != nullptr, "both operands of a half-pair product need the bounds of their rows");
+      TORCH_CHECK(q.a.row0 == 0 && q.b.row0 == 0, "half-pair operands are whole arrays");
       TORCH_CHECK(q.K % kBK == 0, "half-pair operands are padded to a multiple of ", kBK, " along K");
       TORCH_CHECK(half_sym || !(p.flags & kFlagSplitOut) || p.d_lo == nullptr, "a tf32 pair from half pairs needs a symmetric plan");
       if ((p.flags & kFlagSplitOut) && p.d_lo == nullptr) {  // (with a d_lo the output is a tf32 pair)
@@ -237,9 +248,10 @@ class PlanBuilder {
         TORCH_CHECK(!half_sym || (p.flags & kFlagFixedScale), "a symmetric plan's half-pair outputs have a given bound");
         TORCH_CHECK(half_sym || ((p.flags & kFlagNoC) && !(p.flags & (kFlagSumSq | kFlagTrace | kFlagAddDiag))),
                     "a half-pair split output that is more than alpha A B^T needs a symmetric plan");
-        TORCH_CHECK(p.d_hi != nullptr && p.d_meta != nullptr && p.ldd % kBK == 0 && p.ldd >= p.N &&
+        TORCH_CHECK(p.d_hi != nullptr && p.d_bound != nullptr && p.ldd % kBK == 0 && p.ldd >= p.N &&
                         reinterpret_cast<uintptr_t>(p.d_hi) % 16 == 0,
-                    "a half-pair split output needs its meta data, a 16-byte aligned base and a pitch that is a multiple of ", kBK);
+                    "a half-pair split output needs its bounds, a 16-byte aligned base and a pitch that is a multiple of ", kBK);
+        TORCH_CHECK((p.d_left != nullptr) == (p.d_right != nullptr), "the bounds of a result follow from those of both operands");
       }
     } else if (p.flags & kFlagSplitOut) {
       TORCH_CHECK(p.d_hi != nullptr && p.d_lo != nullptr, "split output needs d_hi and d_lo");
@@ -269,9 +281,12 @@ class PlanBuilder {
       const int v = env != nullptr ? std::atoi(env) : 12;
       return v > 0 ? v : 12;
     }();
-    // Half pairs run 128 x 128 or 128 x 256 tiles.  A wide tile takes 1.45 times as long as a narrow one
-    // for twice the work (its B operand is read from shared memory once for twice the rows), but
-    // halves the number of tiles: the width with the lower estimated time per launch is taken.
+    // Half pairs run 128 x 128 or 128 x 256 tiles.  A wide tile takes about 1.7 times as long as a narrow one
+    // for twice the work (its A operand is read from shared memory once for twice the columns, but its
+    // epilogue does not overlap with the next tile), and halves the number of tiles: the width with the lower
+    // estimated time per launch is taken.  Products of a step on one B200, narrow and wide: 2415 and 2103 us over an
+    // 8192 x 8192 weight (ratio per tile 1.74), 8163 and 6545 us over a SOAP layer of 2048 (1.60), 467 and 464 us over two
+    // GPT-2 layers, where a launch has one to two tiles per SM.
     int widest = kBN;
     if (half_) {
       const int sms = at::cuda::getDeviceProperties(device_.index())->multiProcessorCount;
@@ -284,7 +299,7 @@ class PlanBuilder {
           wide += (cols + 1) / 2;
         }
       }
-      if (1.45 * static_cast<double>((wide + sms - 1) / sms) < static_cast<double>((narrow + sms - 1) / sms)) widest = 2 * kBN;
+      if (1.7 * static_cast<double>((wide + sms - 1) / sms) < static_cast<double>((narrow + sms - 1) / sms)) widest = 2 * kBN;
     }
     for (const Order& o : order) {
       const GemmProblem& p = problems_[o.problem];
@@ -313,6 +328,7 @@ class PlanBuilder {
         }
       }
     }
+    for (size_t i = first; i < tiles_.size(); ++i) tiles_[i].bufs = widest > kBN ? 1 : 2;
     if (half_ && !half_sym_) split_along_k(first);
     launch_begin_ = static_cast<int>(problems_.size());
     return {first, static_cast<int64_t>(tiles_.size()) - first};
@@ -326,7 +342,7 @@ class PlanBuilder {
     const size_t table_bytes = problems_.size() * sizeof(GemmProblem);
     const size_t map_bytes = maps_.size() * sizeof(CUtensorMap);
     // [problems][tensor maps][counters of the split tiles: zero][their partial sums]
-    const size_t counter_bytes = (static_cast<size_t>(split_tiles_) * (kBM / 32) * sizeof(int) + 255) / 256 * 256;
+    const size_t counter_bytes = (static_cast<size_t>(split_tiles_) * kCountersPerTile * sizeof(int) + 255) / 256 * 256;
     const size_t host_bytes = table_bytes + map_bytes + counter_bytes;
     auto buffer = torch::empty({static_cast<int64_t>(host_bytes + partial_floats_ * sizeof(float))},
                                torch::dtype(torch::kUInt8).device(device_));
@@ -392,7 +408,7 @@ class PlanBuilder {
         u.part = part;
         u.parts = parts;
         u.partial = reinterpret_cast<float*>(static_cast<uintptr_t>(partial_floats_));  // offsets: see finalize
-        u.counter = reinterpret_cast<int*>(static_cast<uintptr_t>(split_tiles_ * (kBM / 32)));
+        u.counter = reinterpret_cast<int*>(static_cast<uintptr_t>(split_tiles_ * kCountersPerTile));
         out.push_back(u);
       }
       if (parts > 1) {
@@ -446,7 +462,7 @@ struct SpecTensors {
 
 // Spec fields: (a_hi, a_lo | None, b_hi, b_lo | None, c | None, d_hi | None, d_lo | None, sumsq | None,
 //               ldc, ldd, flags, upper_tiles_only [, push_offset [, (a_row0, a_k0, b_row0, b_k0, M, N, K)
-//               [, (a_meta, b_meta, d_meta | None)]]])
+//               [, (a_bound, a_div, b_bound, b_div, d | None)]]]), d = (left | None, right | None, cap | None, bound), see GemmProblem
 // With a view field the operands are views, of the given origin and extent, of the arrays passed.  With the last
 // field the operands and the split output are half pairs (a_lo, b_lo and d_lo are None).
 void add_spec(PlanBuilder& builder, const py::tuple& s, std::vector<std::unique_ptr<SpecTensors>>& keep) {
@@ -494,11 +510,25 @@ void add_spec(PlanBuilder& builder, const py::tuple& s, std::vector<std::unique_
     TORCH_CHECK(g.b_hi.size(1) == q.K, "A and B must agree on K");
   }
   if (s.size() == 15 && !s[14].is_none()) {
-    const auto metas = s[14].cast<std::tuple<torch::Tensor, torch::Tensor, std::optional<torch::Tensor>>>();
-    for (const torch::Tensor* t : {&std::get<0>(metas), &std::get<1>(metas)}) TORCH_CHECK(t->numel() >= 2, "meta data has two entries");
-    q.a_meta = fptr(std::get<0>(metas));
-    q.b_meta = fptr(std::get<1>(metas));
-    q.d_meta = fptr(std::get<2>(metas));
+    using Opt = std::optional<torch::Tensor>;
+    const auto bounds = s[14].cast<std::tuple<torch::Tensor, int64_t, torch::Tensor, int64_t, std::optional<std::tuple<Opt, Opt, Opt, Opt>>>>();
+    auto rows = [](const torch::Tensor& t, int64_t div, int64_t count) -> const float* {
+      TORCH_CHECK(div >= 1 && div < (int64_t{1} << 31) && (count - 1) / div < t.numel() && t.is_contiguous(), "a bound per row, or per group of rows");
+      return fptr(t);
+    };
+    q.a_bound = rows(std::get<0>(bounds), std::get<1>(bounds), q.M);
+    q.b_bound = rows(std::get<2>(bounds), std::get<3>(bounds), q.N);
+    q.a_div = static_cast<int>(std::get<1>(bounds));
+    q.b_div = static_cast<int>(std::get<3>(bounds));
+    if (const auto& d = std::get<4>(bounds); d.has_value()) {
+      for (const Opt* t : {&std::get<0>(*d), &std::get<3>(*d)}) {
+        TORCH_CHECK(!t->has_value() || (*t)->numel() >= (q.flags & kFlagFixedScale ? 1 : q.M), "a bound per row of the result");
+      }
+      q.d_left = fptr(std::get<0>(*d));
+      q.d_right = fptr(std::get<1>(*d));
+      q.d_cap = fptr(std::get<2>(*d));
+      q.d_bound = fptr(std::get<3>(*d));
+    }
   }
   builder.add(q);
 }
@@ -576,7 +606,8 @@ void run_gemm_plan_push(const torch::Tensor& problems, const torch::Tensor& tile
 }
 
 // Block table.  Each spec: (param_view, grad_offset, grad_slot, m, n, n_pad, m_pad, m1, v, mom, z,
-//                           g_hi, g_lo, gt_hi, gt_lo, f_hi, f_lo, p, norms, send_ptr, slot_offset, ev, aux [, meta])
+//                           g_hi, g_lo, gt_hi, gt_lo, f_hi, f_lo, p, norms, send_ptr, slot_offset, ev, aux
+//                           [, (g_rows, g_cols, col_div, f_rows, f_cols, s_rows, s_cols)])
 std::tuple<torch::Tensor, torch::Tensor, int64_t> build_block_table(const std::vector<py::tuple>& specs) {
   std::vector<BlockDesc> blocks(specs.size());
   std::vector<TileRef> tiles;
@@ -620,10 +651,24 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t> build_block_table(const std::v
     b.slot_offset = s[20].cast<int64_t>();
     b.ev = opt(21);
     b.aux = s[22].cast<int>();
+    b.col_div = 1;
     if (s.size() == 24) {
-      const auto meta = s[23].cast<torch::Tensor>();
-      TORCH_CHECK(meta.numel() >= 6 && meta.is_contiguous(), "block meta data has six entries");
-      b.meta = meta.data_ptr<float>();
+      using Opt = std::optional<torch::Tensor>;
+      const auto m = s[23].cast<std::tuple<Opt, Opt, int, Opt, Opt, Opt, Opt>>();
+      auto bounds = [](const Opt& t, int64_t count) -> float* {
+        TORCH_CHECK(!t.has_value() || (t->numel() >= count && t->is_contiguous()), "a bound per row of a half-pair array");
+        return t.has_value() ? fptr(*t) : nullptr;
+      };
+      b.col_div = std::get<2>(m);
+      TORCH_CHECK(b.col_div >= 1, "block bounds");
+      b.g_rows = bounds(std::get<0>(m), b.m);
+      b.g_cols = bounds(std::get<1>(m), (b.n + b.col_div - 1) / b.col_div);
+      b.f_rows = bounds(std::get<3>(m), b.m);
+      b.f_cols = bounds(std::get<4>(m), b.n);
+      b.s_rows = bounds(std::get<5>(m), b.m);
+      b.s_cols = bounds(std::get<6>(m), b.n);
+      TORCH_CHECK((b.g_hi == nullptr || b.g_rows) && (b.gt_hi == nullptr || b.g_cols) && (b.f_hi == nullptr || b.f_rows) &&
+                      (b.ev == nullptr || b.s_rows), "a half-pair array needs the bounds of its rows");
       TORCH_CHECK(b.n_pad % kBK == 0 && b.m_pad % kBK == 0, "half-pair arrays have pitches that are multiples of ", kBK);
     }
   }
@@ -641,6 +686,50 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t> build_block_table(const std::v
 
 inline const TileRef* tile_ptr(const torch::Tensor& tiles) { return reinterpret_cast<const TileRef*>(tiles.data_ptr()); }
 
+// Launch table of row_bounds.  Each spec: (pairs [d, pitch], rows, vec, out, top | None).
+using RowBoundTable = std::tuple<torch::Tensor, torch::Tensor, int64_t>;
+RowBoundTable build_row_bound_table(const std::vector<py::tuple>& specs) {
+  std::vector<RowBoundOp> ops(specs.size());
+  std::vector<int2> bands;
+  torch::Device device(torch::kCPU);
+  for (size_t i = 0; i < specs.size(); ++i) {
+    const py::tuple& s = specs[i];
+    TORCH_CHECK(s.size() == 5, "row bound spec must have 5 fields");
+    const auto mat = s[0].cast<torch::Tensor>();
+    TORCH_CHECK(mat.is_cuda() && mat.scalar_type() == torch::kFloat32 && mat.dim() == 2 && mat.is_contiguous() && mat.size(1) % kBK == 0 &&
+                    mat.size(0) <= mat.size(1) && reinterpret_cast<uintptr_t>(mat.data_ptr()) % 16 == 0,
+                "row bounds are taken of a square array of half pairs");
+    device = mat.device();
+    RowBoundOp& op = ops[i];
+    op.d = static_cast<int>(mat.size(0));
+    op.ld = static_cast<int>(mat.stride(0));
+    op.mat = mat.data_ptr<float>();
+    auto vector = [&](int k) -> float* {
+      const auto t = s[k].cast<torch::Tensor>();
+      TORCH_CHECK(t.numel() >= (k == 2 ? op.ld : op.d) && t.is_contiguous(), "a bound per row, those of columns padded like a row");
+      TORCH_CHECK(k != 2 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "bounds of columns are 16-byte aligned");
+      return fptr(t);
+    };
+    op.rows = vector(1);
+    op.vec = vector(2);
+    op.out = vector(3);
+    op.top = fptr(s[4].cast<std::optional<torch::Tensor>>());
+    for (int r = 0; r < (op.d + kRowBoundRows - 1) / kRowBoundRows; ++r) bands.push_back(make_int2(static_cast<int>(i), r));
+  }
+  auto d_ops = upload_bytes(ops.data(), ops.size() * sizeof(RowBoundOp), device);
+  auto d_bands = upload_bytes(bands.data(), bands.size() * sizeof(int2), device);
+  return {d_ops, d_bands, static_cast<int64_t>(bands.size())};
+}
+
+void row_bounds(const RowBoundTable& table) {
+  LaunchScope scope("ob200::row_bounds");
+  c10::cuda::CUDAGuard guard(std::get<0>(table).device());
+  launch_row_bounds(reinterpret_cast<const RowBoundOp*>(std::get<0>(table).data_ptr()),
+                    reinterpret_cast<const int2*>(std::get<1>(table).data_ptr()), static_cast<int>(std::get<2>(table)),
+                    at::cuda::getCurrentCUDAStream());
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+}
+
 void grad_prologue(const torch::Tensor& blocks, const torch::Tensor& tiles, int64_t num_tiles,
                    const torch::Tensor& grad_ptrs, double l2_weight_decay, double beta1, double beta3,
                    double bias_correction1, int64_t graft_kind, double graft_beta2, double graft_weight,
@@ -648,7 +737,7 @@ void grad_prologue(const torch::Tensor& blocks, const torch::Tensor& tiles, int6
                    int64_t num_grad_peers, double grad_scale, bool filtered_plain, const std::optional<torch::Tensor>& scratch) {
   LaunchScope scope("ob200::grad_prologue");
   c10::cuda::CUDAGuard guard(blocks.device());
-  if (scratch.has_value()) {  // the norms and meta data the step accumulates into start at zero
+  if (scratch.has_value()) {  // the norms and bounds the step accumulates into start at zero
     TORCH_CHECK(scratch->is_cuda() && scratch->is_contiguous(), "step scratch must be a contiguous CUDA tensor");
     C10_CUDA_CHECK(cudaMemsetAsync(scratch->data_ptr(), 0, scratch->nbytes(), at::cuda::getCurrentCUDAStream()));
   }
@@ -1438,15 +1527,17 @@ void transpose_split(const torch::Tensor& ops, const torch::Tensor& tiles, int64
   C10_CUDA_KERNEL_LAUNCH_CHECK();
 }
 
-// Each spec: (src [d, d], dst, dst_t | None, meta): see PairOp.  Returns (ops, bands, number of bands, tiles, number of tiles).
+// Each spec: (src [d, d], dst, (rows, l1 | None, top | None), dst_t | None [, (rows, l1 | None, top | None) of dst_t]): see
+// PairOp.  Returns (ops, bands, number of bands, tiles, number of tiles).
 std::tuple<torch::Tensor, torch::Tensor, int64_t, torch::Tensor, int64_t> build_pair_table(const std::vector<py::tuple>& specs) {
   std::vector<PairOp> ops(specs.size());
   std::vector<int2> bands;
   std::vector<int4> tiles;
   torch::Device device(torch::kCPU);
+  using Opt = std::optional<torch::Tensor>;
   for (size_t i = 0; i < specs.size(); ++i) {
     const py::tuple& s = specs[i];
-    TORCH_CHECK(s.size() == 4, "pair spec must have 4 fields");
+    TORCH_CHECK(s.size() >= 4, "pair spec must have 4 or 5 fields");
     const auto src = s[0].cast<torch::Tensor>();
     TORCH_CHECK(src.is_cuda() && src.scalar_type() == torch::kFloat32 && src.dim() == 2 && src.stride(1) == 1 &&
                     src.size(0) == src.size(1),
@@ -1457,7 +1548,7 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t, torch::Tensor, int64_t> build_
     op.d = static_cast<int>(src.size(0));
     op.ld_src = static_cast<int>(src.stride(0));
     auto take = [&](int k, int* ld) -> float* {
-      const auto t = s[k].cast<std::optional<torch::Tensor>>();
+      const auto t = s[k].cast<Opt>();
       *ld = 0;
       if (!t.has_value()) return nullptr;
       TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->dim() == 2 && t->stride(1) == 1 && t->size(0) >= op.d &&
@@ -1467,13 +1558,21 @@ std::tuple<torch::Tensor, torch::Tensor, int64_t, torch::Tensor, int64_t> build_
       *ld = static_cast<int>(t->stride(0));
       return t->data_ptr<float>();
     };
+    auto take_bounds = [&](int k) -> PairBounds {
+      const auto m = s[k].cast<std::tuple<torch::Tensor, Opt, Opt>>();
+      TORCH_CHECK(std::get<0>(m).numel() >= op.d && (!std::get<1>(m).has_value() || std::get<1>(m)->numel() >= op.d), "a bound per row");
+      return {fptr(std::get<0>(m)), fptr(std::get<1>(m)), fptr(std::get<2>(m))};
+    };
     op.dst = take(1, &op.ld_dst);
-    op.dst_t = take(2, &op.ld_t);
+    op.dst_t = take(3, &op.ld_t);
     TORCH_CHECK(op.dst != nullptr && op.dst_t != op.src, "pair destinations");
     TORCH_CHECK(op.dst != op.src || op.ld_dst == op.ld_src, "a conversion in place keeps the pitch");
-    op.meta = fptr(s[3].cast<std::optional<torch::Tensor>>());
-    TORCH_CHECK(op.meta != nullptr, "pair meta data missing");
-    for (int r = 0; r < (op.d + 7) / 8; ++r) bands.push_back(make_int2(static_cast<int>(i), r));
+    op.of_rows = take_bounds(2);
+    op.of_cols = {};
+    if (op.dst_t != nullptr) op.of_cols = take_bounds(4);
+    const int row_bands = (op.d + 7) / 8, col_bands = op.dst_t != nullptr ? (op.d + 31) / 32 : 0;
+    for (int r = 0; r < row_bands; ++r) bands.push_back(make_int2(static_cast<int>(i), r));
+    for (int c = 0; c < col_bands; ++c) bands.push_back(make_int2(static_cast<int>(i), -1 - c));
     for (int r = 0; r < (op.d + 31) / 32; ++r)
       for (int c = 0; c < (op.d + 31) / 32; ++c) tiles.push_back(make_int4(static_cast<int>(i), r, c, 0));
   }
@@ -1551,6 +1650,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("l2_weight_decay"), py::arg("beta1"), py::arg("beta3"), py::arg("bias_correction1"), py::arg("graft_kind"),
         py::arg("graft_beta2"), py::arg("graft_weight"), py::arg("graft_bc2"), py::arg("graft_eps"), py::arg("write_split"),
         py::arg("status"), py::arg("num_grad_peers"), py::arg("grad_scale"), py::arg("filtered_plain") = false, py::arg("scratch") = std::optional<torch::Tensor>());
+  m.def("build_row_bound_table", &build_row_bound_table);
+  m.def("row_bounds", &row_bounds);
   m.def("direction_epilogue", &direction_epilogue);
   m.def("gathered_apply", &gathered_apply);
   m.def("peer_barrier", &peer_barrier);

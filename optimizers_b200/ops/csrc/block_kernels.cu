@@ -123,40 +123,44 @@ __device__ __forceinline__ float filtered_gradient(float m_old, float m_new, flo
   return f / a.bias_correction1;
 }
 
-// Block-wide maxima of NV values, each added to dst[k] (non-negative floats order like their bits).
-template <int NV>
-__device__ __forceinline__ void atomic_max_block(float (&v)[NV], float* const (&dst)[NV], float (&red)[NV][8]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Maxima over the 32 lanes of a warp of eight values each, with nine shuffles: lane l returns that of value l / 4.
+__device__ __forceinline__ float warp_max8(float (&v)[8]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
+  for (int h = 4; h >= 1; h >>= 1) {
+    const bool upper = (lane & (4 * h)) != 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] = fmaxf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-    if (lane == 0) red[k][warp] = v[k];
+    for (int k = 0; k < h; ++k) {
+      const float send = upper ? v[k] : v[k + h], keep = upper ? v[k + h] : v[k];
+      v[k] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, 4 * h));
+    }
   }
-  __syncthreads();
-  if (threadIdx.x < NV) {
-    float m = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) m = fmaxf(m, red[threadIdx.x][w]);
-    if (m > 0.f && dst[threadIdx.x] != nullptr) atomicMax(reinterpret_cast<int*>(dst[threadIdx.x]), __float_as_int(m));
-  }
-  __syncthreads();
+  v[0] = fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 2));
+  return fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
 }
 
-// Largest |gradient| and |filtered gradient| of every block, for the scale of their fp16 pairs.  Reads what
-// the prologue reads again (at most 12 of its 12 + 20 bytes per element); up to the L2 capacity those
+// Largest value of each of the 128 columns of a tile, found by its eight warps in `cols`, into dst[column / div].
+__device__ __forceinline__ void columns_into(float* dst, const float (&cols)[8][kWide], int j0, int n, int div) {
+  const int j = j0 + static_cast<int>(threadIdx.x) % kWide;
+  if (dst == nullptr || j >= n) return;
+  float m = cols[0][j - j0];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) m = fmaxf(m, cols[w][j - j0]);
+  max_into(dst + j / div, m);
+}
+
+// Largest |gradient| and |filtered gradient| of every row and column, for the scales of their fp16 pairs and of the products'.  Reads what the prologue reads again (at most 12 of its 12 + 20 bytes per element); up to the L2 capacity those
 // second reads do not reach HBM.  The pairs save 16 bytes per element in the prologue itself.  On one B200 the two
-// launches take 129 + 35 us for two GPT-2 layers (142 for the prologue that wrote tf32 pairs), which the
-// products more than give back.
+// launches take 133 + 43 us for two GPT-2 layers (142 for the prologue that wrote tf32 pairs) and 454 + 138 us for an 8192 x
+// 8192 weight, which the products more than give back.
 __global__ void __launch_bounds__(256) grad_amax_kernel(PrologueArgs a) {
-  __shared__ float red[2][8];
+  __shared__ __align__(16) float cols[2][8][kWide];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < a.num_tiles; t += gridDim.x) {
     const TileRef ref = a.tiles[t];
     const BlockDesc& b = a.blocks[ref.block];
-    if (b.aux == 1) continue;  // the block's other view of the same gradient
     const float* src = a.grad_ptrs[b.grad_slot];
-    const int i0 = ref.ti * kTile, j = ref.tj * kWide + 4 * lane;
+    const int i0 = ref.ti * kTile, j0 = ref.tj * kWide, j = j0 + 4 * lane;
     const int cnt = b.n - j < 4 ? b.n - j : 4;
     const bool has_m1 = b.m1 != nullptr, l2 = a.l2_weight_decay != 0.f;
     const bool vec = ((b.n | b.param_pitch | b.grad_offset) & 3) == 0 && aligned16(b.param) && aligned16(b.m1) && aligned16(src);
@@ -178,19 +182,32 @@ __global__ void __launch_bounds__(256) grad_amax_kernel(PrologueArgs a) {
       }
       if (has_m1) load4<false>(mo[r], b.m1 + e, vec, cnt);
     }
-    float top[2] = {0.f, 0.f};
+    float top[8], col[2][4] = {};  // rows of the gradient, then of the filtered gradient
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
+      top[r] = top[4 + r] = 0.f;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float gk = g[r][k];
         const float f = has_m1 ? filtered_gradient(mo[r][k], lerpf(mo[r][k], gk, 1.f - a.beta1), gk, a) : gk;
-        top[0] = fmaxf(top[0], finite_abs(gk));
-        top[1] = fmaxf(top[1], finite_abs(f));
+        const float x = finite_abs(gk);
+        top[r] = fmaxf(top[r], x);
+        col[0][k] = fmaxf(col[0][k], x);
+        top[4 + r] = fmaxf(top[4 + r], finite_abs(f));
+        col[1][k] = fmaxf(col[1][k], finite_abs(f));
       }
     }
-    float* const dst[2] = {b.meta + kMetaGrad, b.meta + kMetaFiltered};
-    atomic_max_block<2>(top, dst, red);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      *reinterpret_cast<float4*>(&cols[s][warp][4 * lane]) = make_float4(col[s][0], col[s][1], col[s][2], col[s][3]);
+    const float mine = warp_max8(top);
+    const int row = i0 + warp + 8 * ((lane >> 2) & 3);
+    float* rows = lane < 16 ? b.g_rows : b.f_rows;
+    if ((lane & 3) == 0 && row < b.m && rows != nullptr) max_into(rows + row, mine);
+    __syncthreads();
+    if (threadIdx.x < kWide) columns_into(b.g_cols, cols[0], j0, b.n, b.col_div);
+    else columns_into(b.f_cols, cols[1], j0, b.n, 1);
+    __syncthreads();
   }
 }
 
@@ -202,6 +219,7 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
   __shared__ __align__(16) float t_hi[kTile][kPair ? kWide : kWide + 1];
   __shared__ float t_lo[kPair ? 1 : kTile][kPair ? 1 : kWide + 1];
   __shared__ float red[8];
+  __shared__ float scale_g[kPair ? kTile : 1], scale_f[kPair ? kTile : 1], scale_t[kPair ? kWide : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_src = a.num_grad_peers > 0 ? a.num_grad_peers : 1;
   const bool peer = a.num_grad_peers > 0;
@@ -218,8 +236,6 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
     const bool l2 = a.l2_weight_decay != 0.f, graft = a.graft_kind != kGraftNone && b.norms != nullptr;
     bool vec = ((b.n | b.param_pitch | b.grad_offset) & 3) == 0 && aligned16(b.param) && aligned16(b.m1) && aligned16(b.v);
     for (int r = 0; r < n_src; ++r) vec = vec && aligned16(srcs[r]);
-    const float scale_g = kPair ? pair_scale(b.meta[kMetaGrad]) : 1.f;
-    const float scale_f = kPair ? pair_scale(b.meta[kMetaFiltered]) : 1.f;
 
     // ---- all loads of the tile first (4 rows x up to 4 arrays in flight per thread)
     float g[4][4], mo[4][4], vo[4][4];
@@ -253,6 +269,18 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
       }
       if (has_m1) load4<false>(mo[r], b.m1 + e, vec, cnt);
       if (has_v) load4<false>(vo[r], b.v + e, vec, cnt);
+    }
+
+    if constexpr (kPair) {  // the scales of the tile's rows and columns, while the loads are in flight
+      const int k = threadIdx.x;
+      if (k < kWide) {
+        if (b.gt_hi != nullptr && j0 + k < b.n) scale_t[k] = pair_scale(b.g_cols[(j0 + k) / b.col_div]);
+      } else if (k < kWide + kTile) {
+        if (b.g_hi != nullptr && i0 + k - kWide < b.m) scale_g[k - kWide] = pair_scale(b.g_rows[i0 + k - kWide]);
+      } else if (k < kWide + 2 * kTile) {
+        if (b.f_rows != nullptr && i0 + k - kWide - kTile < b.m) scale_f[k - kWide - kTile] = pair_scale(b.f_rows[i0 + k - kWide - kTile]);
+      }
+      __syncthreads();
     }
 
     // ---- compute and store
@@ -317,8 +345,8 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
       }
       if (kPair && i < b.m && j < b.n_pad) {  // up to the end of the last chunk: its padding is written as zeros
         const long long row = static_cast<long long>(i) * b.n_pad;
-        if (b.g_hi != nullptr) store_pair4(b.g_hi + row, j, hi, scale_g);
-        if (b.f_hi != nullptr && !a.filtered_plain) store_pair4(b.f_hi + row, j, fh, scale_f);
+        if (b.g_hi != nullptr) store_pair4(b.g_hi + row, j, hi, scale_g[li]);
+        if (b.f_hi != nullptr && !a.filtered_plain) store_pair4(b.f_hi + row, j, fh, scale_f[li]);
       }
       if (kPair && want_t) {
         *reinterpret_cast<float4*>(&t_hi[li][4 * (lane ^ (li >> 2))]) = make_float4(hi[0], hi[1], hi[2], hi[3]);
@@ -343,7 +371,7 @@ __global__ void __launch_bounds__(256, 3) grad_prologue_kernel(PrologueArgs a) {
           if (jj < b.n) {
             const int col = ((lj & ~3) ^ (4 * (threadIdx.x & 7))) + (lj & 3);
             const float h[4] = {t_hi[ii][col], t_hi[ii + 1][col], t_hi[ii + 2][col], t_hi[ii + 3][col]};
-            store_pair4(b.gt_hi + static_cast<long long>(jj) * b.m_pad, i0 + ii, h, scale_g);
+            store_pair4(b.gt_hi + static_cast<long long>(jj) * b.m_pad, i0 + ii, h, scale_t[lj]);
           }
         } else if (jj < b.n && i0 + ii < b.m) {
           const long long o = static_cast<long long>(jj) * b.m_pad + i0 + ii;  // m_pad % 4 == 0
@@ -548,12 +576,60 @@ __global__ void __launch_bounds__(256) gathered_apply_kernel(const BlockDesc* __
   }
 }
 
-// kMeasure: only the largest |S| of each block, into its PairMeta.
+// Four rows per warp; of each 128-byte chunk the 64 bytes of hi halves.  An entry differs from its hi half by 2^-11 of it, or
+// by 2^-25 where that is subnormal.  Bound by reading them (2 bytes per entry of every inverse root once per step): the entries
+// of vec, which a row needs eight of for every 16 bytes, are loaded once for the four.  Sixteen roots of 2048: 53 us (82 with
+// a row per warp).
+__global__ void __launch_bounds__(256) row_bounds_kernel(const RowBoundOp* __restrict__ ops, const int2* __restrict__ bands, int num_bands) {
+  constexpr int kRows = kRowBoundRows / 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int t = blockIdx.x; t < num_bands; t += gridDim.x) {
+    const int2 ref = bands[t];
+    const RowBoundOp op = ops[ref.x];
+    const int row0 = ref.y * kRowBoundRows + warp * kRows;
+    if (row0 >= op.d) continue;
+    const char* src[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+      src[r] = reinterpret_cast<const char*>(op.mat + static_cast<long long>(min(row0 + r, op.d - 1)) * op.ld) + 16 * (lane & 3);
+    const int chunks = op.ld / kPairChunk;
+    float sum[kRows] = {};
+#pragma unroll 4
+    for (int c = lane >> 2; c < chunks; c += 8) {
+      union { uint4 u; __half2 h[4]; } hi[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) hi[r].u = *reinterpret_cast<const uint4*>(src[r] + c * 4 * kPairChunk);
+      const int k0 = c * kPairChunk + 8 * (lane & 3);
+      const float4 lo = __ldg(reinterpret_cast<const float4*>(op.vec + k0)), up = __ldg(reinterpret_cast<const float4*>(op.vec + k0) + 1);
+      const float x[8] = {lo.x, lo.y, lo.z, lo.w, up.x, up.y, up.z, up.w};
+#pragma unroll
+      for (int r = 0; r < kRows; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = __half22float2(__habs2(hi[r].h[k]));
+          sum[r] = fmaf(f.x + 0x1p-25f, x[2 * k], sum[r]);
+          sum[r] = fmaf(f.y + 0x1p-25f, x[2 * k + 1], sum[r]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+      if (lane == 0 && row0 + r < op.d) {
+        const float bound = 1.001f * sum[r] * pair_inverse_scale(op.rows[row0 + r]);
+        op.out[row0 + r] = bound;
+        if (op.top != nullptr) max_into(op.top, bound);
+      }
+    }
+  }
+}
+
+// kMeasure: only the largest |S| of each row and column.
 template <bool kMeasure>
 __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restrict__ blocks,
                                                         const TileRef* __restrict__ tiles, int num_tiles, float bc2,
                                                         float inv_root, float eps, int form) {
-  __shared__ float red[1][8];
+  __shared__ __align__(16) float cols[kMeasure ? 8 : 1][kWide];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
     const TileRef ref = tiles[t];
@@ -564,7 +640,6 @@ __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restr
     const int i0 = ref.ti * kTile, j = ref.tj * kWide + 4 * lane;
     const int cnt = b.n - j < 4 ? b.n - j : 4;
     const bool vec = (b.n & 3) == 0 && aligned16(b.ev) && aligned16(b.p);
-    const float scale = !kMeasure && form == kFormPair ? pair_scale(b.meta[kMetaScaled]) : 1.f;
     float ev[4][4], p[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -576,7 +651,7 @@ __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restr
       load4<false>(ev[r], b.ev + e, vec, cnt);
       load4<false>(p[r], b.p + e, vec, cnt);
     }
-    float top[1] = {0.f};
+    float top[8] = {}, col[4] = {};
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = i0 + warp + 8 * r;
@@ -589,14 +664,15 @@ __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restr
         const float base = ev[r][k] / bc2;
         const float pw = inv_root == 0.5f ? sqrtf(base) : inv_root == 0.25f ? sqrtf(sqrtf(base)) : powf(base, inv_root);
         const float s = k < cnt ? p[r][k] / (pw + eps) : 0.f;
-        top[0] = fmaxf(top[0], finite_abs(s));
+        top[r] = fmaxf(top[r], finite_abs(s));
+        col[k] = fmaxf(col[k], finite_abs(s));
         hi[k] = form == kFormSplit ? tf32_round(s) : s;
         lo[k] = s - hi[k];
       }
       if constexpr (!kMeasure) {
         const long long row = static_cast<long long>(i) * b.n_pad;  // n_pad % 4 == 0
         if (form == kFormPair) {
-          if (j < b.n_pad) store_pair4(b.f_hi + row, j, hi, scale);
+          if (j < b.n_pad) store_pair4(b.f_hi + row, j, hi, pair_scale(b.s_rows[i]));
         } else if (cnt > 0) {
           store4(b.f_hi + row + j, hi, true, 4);
           if (form == kFormSplit) store4(b.f_lo + row + j, lo, true, 4);
@@ -604,8 +680,13 @@ __global__ void __launch_bounds__(256) eig_scale_kernel(const BlockDesc* __restr
       }
     }
     if constexpr (kMeasure) {
-      float* const dst[1] = {b.meta + kMetaScaled};
-      atomic_max_block<1>(top, dst, red);
+      *reinterpret_cast<float4*>(&cols[warp][4 * lane]) = make_float4(col[0], col[1], col[2], col[3]);
+      const float mine = warp_max8(top);
+      const int row = i0 + warp + 8 * ((lane >> 2) & 3);
+      if (lane < 16 && (lane & 3) == 0 && row < b.m) max_into(b.s_rows + row, mine);
+      __syncthreads();
+      if (threadIdx.x < kWide) columns_into(b.s_cols, cols, ref.tj * kWide, b.n, 1);
+      __syncthreads();
     }
   }
 }
@@ -696,6 +777,11 @@ void launch_direction_epilogue(const EpilogueArgs& args, cudaStream_t stream) {
   } else {
     direction_epilogue_kernel<false><<<grid_for(args.num_tiles), 256, 0, stream>>>(args);
   }
+}
+
+void launch_row_bounds(const RowBoundOp* ops, const int2* bands, int num_bands, cudaStream_t stream) {
+  if (num_bands <= 0) return;
+  row_bounds_kernel<<<grid_for(num_bands), 256, 0, stream>>>(ops, bands, num_bands);
 }
 
 void launch_eig_scale(const BlockDesc* blocks, const TileRef* tiles, int num_tiles, float bias_correction2,

@@ -51,12 +51,15 @@ struct BlockDesc {
                           // norms are null) and the epilogue kernels skip it
                           // 2: a block none of whose dims is preconditioned: the prologue writes the
                           // filtered gradient to p and its squared norm to norms[1] itself
-  int pad_;
-  float* meta;            // half pairs: PairMeta of the gradient, the filtered gradient and the scaled
-                          // direction (kMeta*, two floats each), zeroed at the start of the step
+  int col_div;            // columns of one g_cols entry: > 1 where gt_hi is re-viewed with that many rows to one
+  // Half pairs: bounds of the rows of the operand arrays, zeroed at the start of the step and measured in it.
+  float* g_rows;          // [m] largest |gradient| of a row: g_hi
+  float* g_cols;          // [n / col_div] of a column: gt_hi
+  float* f_rows;          // [m] largest |filtered gradient| of a row: f_hi
+  float* f_cols;          // [n] of a column (null unless a chain of products starts from it)
+  float* s_rows;          // [m], [n] of the scaled direction: f_hi between the two halves of the SOAP products
+  float* s_cols;
 };
-
-constexpr int kMetaGrad = 0, kMetaFiltered = 2, kMetaScaled = 4;
 
 // Form of the operand arrays the pointwise kernels write.
 enum OperandForm : int {
@@ -117,9 +120,24 @@ struct EpilogueArgs {
   int send_params;                // 1: what is sent is the updated parameter W + update (communicate_params)
 };
 
+// Bounds of the rows of a product A B^T whose result is stored as half pairs, from the matrix itself: with vec[k] the largest
+// |b_jk| of any j, out[i] = sum_k |a_ik| vec[k] bounds the row i of the result however different its columns' sizes are (a
+// root is largest where the gradient is smallest, so the norms of the two alone may be off by many decades), and top the
+// whole.  A is a square array of half pairs, of which the hi halves are read.
+struct RowBoundOp {
+  const float* mat;   // [d, ld] half pairs
+  const float* rows;  // [d] their bounds
+  const float* vec;   // [ld], 16-byte aligned, zero from d on
+  float* out;         // [d]
+  float* top;         // the largest of out, may be null; zeroed by the caller
+  int d, ld;
+};
+constexpr int kRowBoundRows = 32;  // rows of a band
+void launch_row_bounds(const RowBoundOp* ops, const int2* bands, int num_bands, cudaStream_t stream);
+
 // eig_scale: S = P / ((ev / bc2)^(1/root) + eps) on the projected filtered gradient held in
 // BlockDesc::p, written as the operand of the unprojection GEMMs into f_hi / f_lo; with half pairs a
-// first launch finds the largest |S| of each block, from which the pairs' scale follows
+// first launch finds the largest |S| of each row and column, from which the scales follow
 // (reference: shampoo_preconditioner_list.py:1920-1942).
 void launch_eig_scale(const BlockDesc* blocks, const TileRef* tiles, int num_tiles, float bias_correction2,
                       float inv_root, float epsilon, int form, cudaStream_t stream);
@@ -138,7 +156,7 @@ constexpr int kErrPeerTimeout = 4;  // a bounded wait on a peer's flag expired
 void launch_peer_barrier(int* local_flags, const unsigned long long* peer_flag_bases, int my_rank, int world,
                          int seq, int* status, cudaStream_t stream);
 
-// kFormPair: two launches, the first of which finds the largest gradient and filtered gradient of each block.
+// kFormPair: two launches, the first of which finds the largest gradient and filtered gradient of each row and column.
 void launch_grad_prologue(const PrologueArgs& args, cudaStream_t stream);
 void launch_direction_epilogue(const EpilogueArgs& args, cudaStream_t stream);
 

@@ -727,32 +727,58 @@ __global__ void __launch_bounds__(256) transpose_split_kernel(const TransposeOp*
   }
 }
 
-// A warp per row.  The row norm bounds the products' results more tightly than the largest entry does, and
-// with it the scale of a chained product's output.
+// Bands of eight rows, a warp each, and (band index below zero) of 32 columns, a lane each with the rows dealt out to the
+// warps.  Sums are taken in a fixed order, so the bounds, and with them the scales, repeat exactly.
 __global__ void __launch_bounds__(256) pair_measure_kernel(const PairOp* __restrict__ ops, const int2* __restrict__ bands,
                                                            int num_bands) {
+  __shared__ float tops[8][32], sums[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto emit = [](const PairBounds& to, int row, float top, float sum) {
+    to.rows[row] = top;
+    if (to.l1 != nullptr) to.l1[row] = sum;
+    if (to.top != nullptr) max_into(to.top, sum);
+  };
   for (int t = blockIdx.x; t < num_bands; t += gridDim.x) {
     const int2 ref = bands[t];
     const PairOp op = ops[ref.x];
-    const int row = ref.y * 8 + warp;
-    if (row >= op.d) continue;
-    const float* src = op.src + static_cast<long long>(row) * op.ld_src;
-    float top = 0.f, sq = 0.f;
-    for (int j = lane; j < op.d; j += 32) {
-      const float x = finite_abs(src[j]);
-      top = fmaxf(top, x);
-      sq = fmaf(x, x, sq);
-    }
+    float top = 0.f, sum = 0.f;
+    if (ref.y >= 0) {
+      const int row = ref.y * 8 + warp;
+      if (row >= op.d) continue;
+      const float* src = op.src + static_cast<long long>(row) * op.ld_src;
+      for (int j = lane; j < op.d; j += 32) {
+        const float x = finite_abs(src[j]);
+        top = fmaxf(top, x);
+        sum += x;
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      for (int o = 16; o > 0; o >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      }
+      if (lane == 0) emit(op.of_rows, row, top, sum);
+      continue;
     }
-    if (lane == 0 && top > 0.f) {
-      atomicMax(reinterpret_cast<int*>(op.meta), __float_as_int(top));
-      atomicMax(reinterpret_cast<int*>(op.meta + 1), __float_as_int(sq));
+    const int col = 32 * (-1 - ref.y) + lane;
+    if (col < op.d) {
+      for (int i = warp; i < op.d; i += 8) {
+        const float x = finite_abs(op.src[static_cast<long long>(i) * op.ld_src + col]);
+        top = fmaxf(top, x);
+        sum += x;
+      }
     }
+    tops[warp][lane] = top;
+    sums[warp][lane] = sum;
+    __syncthreads();
+    if (warp == 0 && col < op.d) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) {
+        top = fmaxf(top, tops[w][lane]);
+        sum += sums[w][lane];
+      }
+      emit(op.of_cols, col, top, sum);
+    }
+    __syncthreads();
   }
 }
 
@@ -770,12 +796,13 @@ __global__ void __launch_bounds__(256) pair_convert_kernel(const PairOp* __restr
       tile[k][tx] = (r < op.d && c < op.d) ? op.src[static_cast<long long>(r) * op.ld_src + c] : 0.f;
     }
     __syncthreads();
-    const float s = pair_scale(op.meta[0]);
     if (r0 + row < op.d) {
+      const float s = pair_scale(op.of_rows.rows[r0 + row]);
       const float v[4] = {tile[row][g], tile[row][g + 1], tile[row][g + 2], tile[row][g + 3]};
       store_pair4(op.dst + static_cast<long long>(r0 + row) * op.ld_dst, c0 + g, v, s);
     }
     if (op.dst_t != nullptr && c0 + row < op.d) {
+      const float s = pair_scale(op.of_cols.rows[c0 + row]);
       const float v[4] = {tile[g][row], tile[g + 1][row], tile[g + 2][row], tile[g + 3][row]};
       store_pair4(op.dst_t + static_cast<long long>(c0 + row) * op.ld_t, r0 + g, v, s);
     }

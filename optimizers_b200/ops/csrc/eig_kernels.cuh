@@ -134,13 +134,18 @@ void launch_transpose_split(const TransposeOp* ops, const int4* tiles, int num_t
 
 // Operand mirrors as scaled fp16 pairs (half_pair.cuh): dst = the d x d matrix at src (dst may be src: each
 // 32 x 32 tile is replaced by its own chunks), dst_t (may be null) its transpose.  A first launch over
-// 8-row bands finds the largest entry and the largest row norm and puts them into `meta`, which the
-// caller has zeroed.
+// 8-row and 32-column bands finds the largest entry of every row (of every column, for dst_t), which the scales follow, and
+// the 1-norms, from which the bounds of a chained product's rows follow.
+struct PairBounds {
+  float* rows;  // [d] largest |entry| of a row
+  float* l1;    // [d] 1-norms, may be null
+  float* top;   // the largest 1-norm, may be null; zeroed by the caller
+};
 struct PairOp {
   const float* src;
   float* dst;
   float* dst_t;
-  float* meta;
+  PairBounds of_rows, of_cols;  // of the rows of dst and of dst_t
   int d, ld_src, ld_dst, ld_t;
 };
 void launch_pair_mirrors(const PairOp* ops, const int2* bands, int num_bands, const int4* tiles, int num_tiles,

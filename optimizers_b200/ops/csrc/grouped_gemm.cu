@@ -14,8 +14,6 @@ namespace ob200 {
 
 namespace {
 
-constexpr int kThreads = 192;
-constexpr int kEpilogueWarps = 4;
 constexpr int kTileBytesA = kBM * kBK * 4;  // 16 KiB
 constexpr int kTileBytesB = kBN * kBK * 4;  // 16 KiB
 constexpr int kStagePitch = 33;             // floats per staged row: conflict-free transposition
@@ -25,8 +23,14 @@ constexpr uint32_t kIdescHalf = make_idesc(/*f16*/ 0, kBM, 0);  // N is filled i
 template <int kMode>
 struct Cfg {
   static constexpr bool kHalf = kMode == kGemmHalfPair || kMode == kGemmHalfPairSym;
-  static constexpr int kAccCols = kHalf ? 2 * kBN : kBN;  // columns of one accumulator buffer
-  static constexpr int kTmemCols = 2 * kAccCols;                           // two accumulator buffers
+  // Columns of one of two accumulator buffers (half pairs: main and cross sums of a tile of 128 columns).
+  static constexpr int kAccCols = kHalf ? 2 * kBN : kBN;
+  static constexpr int kTmemCols = 2 * kAccCols;
+  // Half pairs: two warps per 32-row stripe, which take its 32-column chunks in turn.  With one accumulator buffer the
+  // MMAs wait for the epilogue.
+  static constexpr int kColumnGroups = kHalf ? 2 : 1;
+  static constexpr int kEpilogueWarps = 4 * kColumnGroups;
+  static constexpr int kThreads = 64 + 32 * kEpilogueWarps;
   // tf32x3: hi and lo of both operands; half pairs: one A tile and up to two B tiles (256 columns)
   static constexpr int kStageBytes =
       kMode == kGemmTf32x3 ? 2 * (kTileBytesA + kTileBytesB) : kTileBytesA + (kHalf ? 2 : 1) * kTileBytesB;
@@ -117,9 +121,14 @@ __device__ __forceinline__ void half_pair_chunk(float (&v)[32], float* st, float
         if (j < count) dst[j] = v[j];
     }
   };
+  auto store_d = [&](float* dst) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= scale;
+    store_pair_chunk(dst, v);
+  };
   if (live) {
     if (write_c) store_c(crow, N - col0, vec);
-    store_pair_chunk(Dhi + static_cast<long long>(row) * ldd + col0, v, scale);
+    store_d(Dhi + static_cast<long long>(row) * ldd + col0);
   }
   if (mirror) {
 #pragma unroll
@@ -128,7 +137,7 @@ __device__ __forceinline__ void half_pair_chunk(float (&v)[32], float* st, float
     if (trow < N) {
       const bool tvec = row0 + 32 <= M && (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(Cp) & 15) == 0;
       if (write_c) store_c(Cp + static_cast<long long>(trow) * ldc + row0, M - row0, tvec);
-      store_pair_chunk(Dhi + static_cast<long long>(trow) * ldd + row0, v, scale);
+      store_d(Dhi + static_cast<long long>(trow) * ldd + row0);
     }
     __syncwarp();
   }
@@ -137,7 +146,7 @@ __device__ __forceinline__ void half_pair_chunk(float (&v)[32], float* st, float
 // kPush: instantiation whose epilogue also stores into the peers' gather buffers; kept apart so
 // that the store loop of the common instantiation is not burdened with it.
 template <int kMode, bool kPush>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Cfg<kMode>::kThreads, 1)
 grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __restrict__ tiles, int num_tiles,
                     float alpha, float beta, float gamma, int* __restrict__ status, const PeerPush push) {
   using C = Cfg<kMode>;
@@ -155,6 +164,9 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
   uint64_t* acc_empty = acc_full + 2;        // [2]
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  float* norm_parts = reinterpret_cast<float*>(tmem_holder + 2);                 // [4][kEpilogueWarps]
+  int* norm_arrived = reinterpret_cast<int*>(norm_parts + 4 * C::kEpilogueWarps);  // [4]
+  static_assert((2 * kStages + 4) * 8 + 8 + 4 * (4 * C::kEpilogueWarps + 4) <= C::kBarrierBytes, "barrier region");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -166,9 +178,10 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], kEpilogueWarps);
+      mbar_init(&acc_empty[b], C::kEpilogueWarps);
     }
     *abort_flag = 0;
+    for (int k = 0; k < 4; ++k) norm_arrived[k] = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
@@ -223,10 +236,11 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       int it = 0;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
         const GemmTile tile = tiles[t];
-        const int buf = it & 1;
-        if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) break;
+        const int buf = tile.bufs == 1 ? 0 : it & 1, round = tile.bufs == 1 ? it : it >> 1;
+        if (!mbar_wait(&acc_empty[buf], (round & 1) ^ 1, abort_flag)) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * C::kAccCols;
+        const uint32_t d_cross = d_tmem + (tile.bufs == 1 ? 2 * kBN : kBN);  // half pairs
         // Columns beyond N are not multiplied (in steps of 16); the epilogue does not read them.
         const int live = kHalf ? min(tile.cols, (problems[tile.problem].N - tile.n0 + 15) & ~15) : kBN;
         const uint32_t idesc_half = kIdescHalf | (static_cast<uint32_t>(live >> 3) << 17);
@@ -241,13 +255,14 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           const uint64_t b_hi = make_kmajor_sw128_desc(s + kTileBytesA);
           if constexpr (kHalf) {
             // A row is [32 fp16 hi | 32 fp16 lo]: K steps of 16 at byte offsets 0 and 32, the lo
-            // halves 64 bytes further.
+            // halves 64 bytes further.  lo is held times 2^11, so its products have their own accumulator.
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               const uint64_t hi = static_cast<uint64_t>(k * 2), lo = static_cast<uint64_t>(4 + k * 2);
-              umma_f16(d_tmem, a_hi + lo, b_hi + hi, idesc_half, kb != tile.kb0 || k != 0);
-              umma_f16(d_tmem, a_hi + hi, b_hi + hi, idesc_half, 1);
-              umma_f16(d_tmem, a_hi + hi, b_hi + lo, idesc_half, 1);
+              const uint32_t first = kb != tile.kb0 || k != 0;
+              umma_f16(d_cross, a_hi + lo, b_hi + hi, idesc_half, first);
+              umma_f16(d_tmem, a_hi + hi, b_hi + hi, idesc_half, first);
+              umma_f16(d_cross, a_hi + hi, b_hi + lo, idesc_half, 1);
             }
             umma_commit(&empty_bar[stage]);
             if (++stage == kStages) {
@@ -284,6 +299,8 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
   } else {
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
+    constexpr int kGroups = C::kColumnGroups;
+    const int group = (warp - 2) >> 2;  // of the stripe's chunks this warp takes group, group + kGroups, ...
     float* st = staging + (warp - 2) * 32 * kStagePitch;
     int it = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
@@ -294,31 +311,74 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       float* __restrict__ Dhi = p->d_hi;
       float* __restrict__ Dlo = p->d_lo;
       const int ldc = p->ldc, ldd = p->ldd;
+      const int row0 = tile.m0 + q * 32;
       const bool do_push = kPush && (flags & kFlagPeerPush) && push.num_peers > 0;
       const long long push_offset = p->push_offset;
-      const int buf = it & 1;
-      if (!mbar_wait(&acc_full[buf], (it >> 1) & 1, abort_flag)) break;
-      tc_fence_after_sync();
-      const int row0 = tile.m0 + q * 32;
-      float sq = 0.f, tr = 0.f;
-      // Half pairs: the accumulator holds (s_a a)(s_b b); the powers of two are taken out one after the
-      // other, since their product may leave the range of fp32.  The scale of a split output follows
-      // from |c_ij| <= ||a_i|| ||b_j||, the same for every tile, so whoever is here writes it.
-      float inv_a = 1.f, inv_b = 1.f, scale_d = 1.f;
-      if constexpr (kHalf) {
-        inv_a = pair_inverse_scale(p->a_meta[0]);
-        inv_b = pair_inverse_scale(p->b_meta[0]);
-        if (kSym && (flags & kFlagSplitOut) && (flags & kFlagFixedScale)) {
-          scale_d = pair_scale(p->d_meta[0]);
-        } else if ((flags & kFlagSplitOut) && Dlo == nullptr) {
-          const float bound = fabsf(alpha) * pair_row_bound(p->a_meta, p->K) * pair_row_bound(p->b_meta, p->K);
-          scale_d = pair_scale(bound);
-          if (threadIdx.x == 64) {
-            p->d_meta[0] = bound;
-            p->d_meta[1] = 0.f;
-          }
+      const int buf = tile.bufs == 1 ? 0 : it & 1, round = tile.bufs == 1 ? it : it >> 1;
+      if (kHalf && beta != 0.f && row0 + lane < M && ((flags & kFlagPackedC) || !(flags & kFlagNoC))) {
+        // The old values of C are on their way to the L2 while the products run.
+        const int row = row0 + lane;
+        const float* crow = (flags & kFlagPackedC) ? Cp + static_cast<long long>(row) * N - (static_cast<long long>(row) * (row + 1)) / 2
+                                                   : Cp + static_cast<long long>(row) * ldc;
+        for (int c = group; c < tile.cols / 32 && tile.n0 + c * 32 < N; c += kGroups) {
+          const int last = min(tile.n0 + c * 32 + 31, N - 1);  // (a row segment may straddle two lines: the first and the last entry)
+          const int first = (flags & kFlagPackedC) ? max(tile.n0 + c * 32, row) : tile.n0 + c * 32;
+          if (first > last) continue;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + first));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + last));
         }
       }
+      // Half pairs: the accumulator will hold (s_a a)(s_b b), with a scale per row of A and of B.  The bound of a row of a
+      // split output is the same for every tile of the row, so whoever is here writes it.  All of it is
+      // fetched before the wait for the products.
+      constexpr int kOwn = kHalf ? 2 * kBN / 32 / kGroups : 1;  // chunks of a stripe that are this warp's
+      float inv_a = 1.f, scale_d = 1.f, inv_cols[kOwn];
+      if constexpr (kHalf) {
+        const int row = min(row0 + lane, M - 1);
+        inv_a = pair_inverse_scale(p->a_bound[row / p->a_div]);
+        if (kSym && (flags & kFlagSplitOut) && (flags & kFlagFixedScale)) {
+          scale_d = pair_scale(p->d_bound[0]);
+        } else if ((flags & kFlagSplitOut) && Dlo == nullptr) {
+          float bound;
+          if (p->d_left != nullptr) {
+            bound = p->d_left[row] * p->d_right[0];
+            if (p->d_cap != nullptr) bound = fminf(bound, p->d_cap[0]);
+            bound *= fabsf(alpha);
+            if (group == 0 && row0 + lane < M) p->d_bound[row] = bound;
+          } else {
+            bound = p->d_bound[row];
+          }
+          scale_d = pair_scale(bound);
+        }
+#pragma unroll
+        for (int k = 0; k < kOwn; ++k)
+          inv_cols[k] = pair_inverse_scale(p->b_bound[min(tile.n0 + (group + k * kGroups) * 32 + lane, N - 1) / p->b_div]);
+      }
+      if (!mbar_wait(&acc_full[buf], round & 1, abort_flag)) break;
+      tc_fence_after_sync();
+      const uint32_t acc_tmem = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols;
+      // The 32 columns of chunk c; with half pairs the cross sums, held times 2^11, join the main ones here.
+      auto load_chunk = [&](int c, float(&v)[32]) {
+        if constexpr (kHalf) {
+          float x[32];
+          tmem_ld_2x32x32(acc_tmem + c * 32, acc_tmem + (tile.bufs == 1 ? 2 * kBN : kBN) + c * 32, v, x);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = fmaf(x[j], kPairLoInv, v[j]);
+        } else {
+          tmem_ld_32x32(acc_tmem + c * 32, v);
+        }
+      };
+      // The accumulator goes back to the MMAs once the warp has loaded its last chunk: with one buffer they wait for it.
+      // (Loading each chunk ahead of the stores of the one before spilled 600 bytes: 2123 -> 2475 us in a step's products over
+      // 8192 x 8192.)
+      bool held = true;
+      auto release = [&]() {
+        if (!held) return;
+        held = false;
+        tc_fence_before_sync();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      };
+      float sq = 0.f, tr = 0.f;
       // Symmetric result (kFlagMirror): only entries on or above the diagonal are taken from the
       // accumulator; every 32 x 32 chunk strictly above the diagonal is also stored transposed and
       // the chunks on the diagonal are symmetrised, so the stored matrix is symmetric bit for bit
@@ -331,49 +391,80 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
       const int chunks = kHalf ? tile.cols / 32 : kBN / 32;
       if (parted && row0 < M) {
         float4* own = stripe_of(tile, tile.part, q) + lane;
-        for (int c = 0; c < chunks && tile.n0 + c * 32 < N; ++c) {
+        for (int c = group; c < chunks && tile.n0 + c * 32 < N; c += kGroups) {
           if ((flags & kFlagPackedC) && tile.n0 + c * 32 + 31 < row0) continue;
           float v[32];
-          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
+          load_chunk(c, v);
 #pragma unroll
           for (int g = 0; g < 8; ++g) own[(c * 8 + g) * 32] = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
         }
+        release();
         __threadfence();
         __syncwarp();
         int arrived = 0;
-        if (lane == 0) arrived = atomicAdd(tile.counter + q, 1);
+        int* counter = tile.counter + q * kGroups + group;
+        if (lane == 0) arrived = atomicAdd(counter, 1);
         finish = __shfl_sync(0xffffffffu, arrived, 0) == tile.parts - 1;
         if (finish) {
-          if (lane == 0) tile.counter[q] = 0;
+          if (lane == 0) *counter = 0;
           __threadfence();
         }
       }
       if (finish) {
+        // Chunks this warp stores: neither beyond N, nor strictly below the diagonal of a packed result, nor written as
+        // the transpose of another.
+        auto next_chunk = [&](int c) {
+          while (c < chunks && (((flags & kFlagPackedC) && tile.n0 + c * 32 + 31 < row0) || (diag_tile && c < q))) c += kGroups;
+          return tile.n0 + c * 32 < N ? c : chunks;
+        };
+        int after;
+        // Exponents of the scales to take out: where no product of two of them leaves the range of fp32, they are
+        // multiplied first.
+        int a_min = 0, a_max = 0;
+        if constexpr (kHalf) {
+          const int e = static_cast<int>(__float_as_uint(inv_a) >> 23) - 127;
+          a_min = __reduce_min_sync(0xffffffffu, e);
+          a_max = __reduce_max_sync(0xffffffffu, e);
+        }
 #pragma unroll 1
-        for (int c = 0; c < chunks; ++c) {
+        for (int c = next_chunk(group); c < chunks; c = after) {
           const int col0 = tile.n0 + c * 32;
-          if (col0 >= N) break;
-          if ((flags & kFlagPackedC) && col0 + 31 < row0) continue;  // chunk strictly below the diagonal
-          if (diag_tile && c < q) continue;  // written as the transpose of chunk (c, q)
+          after = next_chunk(c + kGroups);
           const bool mirror = sym && (!diag_tile || c > q);
           const bool diag_chunk = diag_tile && c == q;
           float v[32];
           if (kMode == kGemmHalfPair && parted) {
             sum_parts(tile, q, c, lane, v);
           } else {
-            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * C::kAccCols + c * 32, v);
+            load_chunk(c, v);
+            if (after >= chunks) release();
           }
           float sq_chunk = 0.f;
           if constexpr (kHalf) {
+            float mine = inv_cols[0];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = (v[j] * inv_a) * inv_b;
-            if (!kSym && (flags & kFlagSplitOut)) {
+            for (int k = 1; k < kOwn; ++k) mine = c == group + k * kGroups ? inv_cols[k] : mine;
+            const int e = static_cast<int>(__float_as_uint(mine) >> 23) - 127;
+            const bool split_out = !kSym && (flags & kFlagSplitOut);
+            if (a_min + __reduce_min_sync(0xffffffffu, e) >= -120 && a_max + __reduce_max_sync(0xffffffffu, e) <= 120) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] *= inv_a * __shfl_sync(0xffffffffu, mine, j);
+            } else {  // one after the other, the smaller first
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float inv_b = __shfl_sync(0xffffffffu, mine, j);
+                v[j] = (v[j] * fminf(inv_a, inv_b)) * fmaxf(inv_a, inv_b);
+              }
+            }
+            if (split_out) {
               // One thread owns the 128-byte chunk of its row: 32 hi, then 32 lo (zero beyond N, which
               // the next product reads as K padding).
               if (row0 + lane < M) {
+                const float factor = alpha * scale_d;
+                const int cols = N - col0;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = col0 + j < N ? alpha * v[j] : 0.f;
-                store_pair_chunk(Dhi + static_cast<long long>(row0 + lane) * ldd + col0, v, scale_d);
+                for (int j = 0; j < 32; ++j) v[j] = j < cols ? factor * v[j] : 0.f;
+                store_pair_chunk(Dhi + static_cast<long long>(row0 + lane) * ldd + col0, v);
               }
               continue;
             }
@@ -579,12 +670,29 @@ grouped_gemm_kernel(const GemmProblem* __restrict__ problems, const GemmTile* __
           sq += sq_chunk;
         }
       }
-      tc_fence_before_sync();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      release();
       if (flags & kFlagSumSq) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0 && sq != 0.f) atomicAdd(p->sumsq, sq);
+        if constexpr (kMode == kGemmHalfPair) {
+          // The warps' sums in a fixed order, by the warp that arrives last (none waits; a warp is at most two tiles ahead
+          // of another): a problem of one tile adds up the same way in every run.
+          if (lane == 0) {
+            float* mine = norm_parts + (it & 3) * C::kEpilogueWarps;
+            mine[warp - 2] = sq;
+            __threadfence_block();
+            if (atomicAdd(&norm_arrived[it & 3], 1) == C::kEpilogueWarps - 1) {
+              norm_arrived[it & 3] = 0;
+              __threadfence_block();
+              float total = 0.f;
+#pragma unroll
+              for (int w = 0; w < C::kEpilogueWarps; ++w) total += static_cast<volatile float*>(mine)[w];
+              if (total != 0.f) atomicAdd(p->sumsq, total);
+            }
+          }
+        } else if (lane == 0 && sq != 0.f) {
+          atomicAdd(p->sumsq, sq);
+        }
       }
       if (flags & kFlagTrace) {
 #pragma unroll
@@ -621,7 +729,7 @@ void launch_impl(const GemmProblem* problems, const GemmTile* tiles, int num_til
     configured = true;
   }
   const int grid = num_tiles < max_ctas ? num_tiles : max_ctas;
-  grouped_gemm_kernel<kMode, kPush><<<grid, kThreads, C::kSmemBytes, stream>>>(problems, tiles, num_tiles, alpha,
+  grouped_gemm_kernel<kMode, kPush><<<grid, C::kThreads, C::kSmemBytes, stream>>>(problems, tiles, num_tiles, alpha,
                                                                                beta, gamma, status, push);
 }
 

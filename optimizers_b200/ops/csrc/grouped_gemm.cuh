@@ -5,21 +5,22 @@
 // with hi = tf32_round(x), lo = x - hi, and every K step issues three tf32 products
 // (hi*hi + hi*lo + lo*hi) into the same fp32 TMEM accumulator, which restores fp32-grade
 // accuracy.  kGemmTf32: one tf32 product on the raw fp32 operands.  kGemmHalfPair: the same three
-// products at the fp16 rate, twice that of tf32, on interleaved scaled fp16 pairs (half_pair.cuh):
+// products at the fp16 rate, twice that of tf32, on interleaved fp16 pairs with a scale per row (half_pair.cuh):
 // hi and lo of 32 consecutive K elements share one 128-byte swizzle row, so an operand is one array of
-// 4 bytes per element, half of the tf32 pair's.  Both splits carry 11 + 11 significant bits; the
-// fp16 one rounds lo where the tensor core truncates a tf32 lo, and sums 16 products instead of 8
-// before each (truncating) accumulation, so its error is the smaller one.  Measured on one B200 (the three
-// products counted): 16 products of 2048^3 in 581 us instead of 1128 (1420 TFLOP/s against 730; cuBLAS bf16
-// reaches 1590), 6 of 768^3 in 27 us instead of 42, relative error against fp64 at K = 2048 7.2e-6 instead
-// of 1.4e-5.
+// 4 bytes per element, half of the tf32 pair's.  Both splits carry 11 + 11 significant bits: a tf32 pair at any
+// size of the entry, an fp16 pair down to 2^-28 of its row's bound.  lo is stored times 2^11, so the two
+// cross products go to an accumulator of their own and join the main one in the epilogue.  The fp16 split
+// rounds lo where the tensor core truncates a tf32 lo, and sums 16 products instead of 8 before each (truncating)
+// accumulation, so over rows whose entries lie within that range its error is the smaller one.  Measured on one
+// B200 (the three products counted): 16 products of 2048^3 in 617 us instead of 1147 (1340 TFLOP/s against 720; cuBLAS
+// bf16 reaches 1640), 6 of 768^3 in 31.5 us instead of 47, relative error against fp64 at K = 2048 2.5e-6 instead of 1.4e-5.
 //
-// Structure (one persistent CTA per SM, 192 threads):
+// Structure (one persistent CTA per SM, 192 threads, 320 with half pairs):
 //   warp 0      TMA producer: cp.async.bulk.tensor tiles of 128 rows x 128 bytes, 128-byte swizzle
 //   warp 1      MMA issuer: tcgen05.mma 128x128x8 kind::tf32, or 128x128x16 / 128x256x16 kind::f16,
 //               accumulators in TMEM, two accumulator buffers so the epilogue of one tile overlaps
-//               the next tile's MMAs
-//   warps 2..5  epilogue: tcgen05.ld, transpose through shared memory, then coalesced global
+//               the next tile's MMAs (half pairs with 256 columns: main and cross accumulators fill the TMEM, one buffer)
+//   warps 2..   epilogue (four warps, eight with half pairs): tcgen05.ld, transpose through shared memory, then coalesced global
 //               access with the fused options below.
 //
 // Epilogue options per problem (flags):
@@ -62,8 +63,8 @@ constexpr int kFlagPeerPush = 32;   // also store the result, cast to the commun
                                     // all-gather of the search directions happens tile by tile from
                                     // the epilogue of the GEMM that produces them
 
-constexpr int kFlagFixedScale = 512;  // half-pair split output: the caller has set the bound in d_meta; needed where
-                                      // the result is more than alpha A B^T
+constexpr int kFlagFixedScale = 512;  // half-pair split output: one bound for all rows, set by the caller in d_bound[0]; needed
+                                      // where the result is more than alpha A B^T
 
 constexpr int kErrPipelineTimeout = 1;  // a bounded mbarrier wait expired
 
@@ -85,10 +86,19 @@ struct alignas(128) GemmProblem {
   int ldc;  // row pitch of C in elements (full mode); N in packed mode
   int ldd;  // row pitch of d_hi / d_lo
   int flags;
-  // kGemmHalfPair: PairMeta of the operands (read) and of the split output (written, kFlagSplitOut)
-  const float* a_meta;
-  const float* b_meta;
-  float* d_meta;
+  // kGemmHalfPair: bounds behind the scales of the operands' rows, that of row r at a_bound[r / a_div] (a re-viewed
+  // array has several view rows per row it was written with; one bound for all rows has a div beyond any row).
+  const float* a_bound;
+  const float* b_bound;
+  int a_div, b_div;
+  // Bounds of the rows of a split output.  d_left null: d_bound[i] is given (RowBoundOp in block_kernels.cuh; kFlagFixedScale:
+  // d_bound[0], for every row).  Else they follow from |sum_k a_ik b_jk| <= |a_i|_1 max|b|, or max|a_i| times the largest
+  // |b_j|_1, and the epilogue writes them: d_bound[i] = |alpha| min(d_left[i] d_right[0], d_cap[0]), d_cap a bound of the
+  // whole result or null.
+  const float* d_left;
+  const float* d_right;
+  const float* d_cap;
+  float* d_bound;
   long long push_offset;  // byte offset of the problem's slot inside the gather buffers (kFlagPeerPush)
 };
 
@@ -101,24 +111,28 @@ struct PeerPush {
 };
 
 // One work item: an output tile, or with parts > 1 the share [kb0, kb1) of its K blocks.  Every part leaves its
-// accumulator at `partial` (part-major, kBM x cols floats each); of each 32-row stripe the warp that arrives
-// last at counter[stripe] adds the parts up in their order, so that the result does not depend on the
+// accumulator at `partial` (part-major, kBM x cols floats each); of each 32-row stripe and half of its 32-column chunks the
+// warp that arrives last at its counter adds the parts up in their order, so that the result does not depend on the
 // arrival, and runs the epilogue on the sum.  No part waits for another.
 struct alignas(16) GemmTile {
   int problem;
   int m0;  // first row of the tile
   int n0;  // first column of the tile
-  int cols;  // 128, or 256 (kGemmHalfPair only)
+  int cols;  // 128, or 256 (half pairs only)
   int kb0, kb1;
   int part, parts;
   float* partial;
-  int* counter;  // [kBM / 32], zero between launches
+  int* counter;  // [kCountersPerTile], zero between launches
+  int bufs;      // accumulator buffers in use, the same for all tiles of a launch: 1 where a tile has 256 columns
+  int pad_[3];
 };
 
 // kGemmHalfPairSym: kGemmHalfPair with the epilogues of the symmetric iterations (split outputs with a given bound,
 // mirrored, with beta, diagonal, norm and trace); an instantiation of its own, so that their registers do
 // not weigh on the step's products.
 enum GemmMode : int { kGemmTf32 = 0, kGemmTf32x3 = 1, kGemmHalfPair = 2, kGemmHalfPairSym = 3 };
+
+constexpr int kCountersPerTile = 8;  // one per 32-row stripe and epilogue warp of it
 
 constexpr int kBM = 128;
 constexpr int kBN = 128;

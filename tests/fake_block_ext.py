@@ -27,11 +27,17 @@ def _at(address, numel, dtype=torch.float32):
 
 class _Block:
     __slots__ = ("param", "grad_offset", "grad_slot", "m", "n", "n_pad", "m_pad", "m1", "v", "mom", "z", "g_hi", "g_lo",
-                 "gt_hi", "gt_lo", "f_hi", "f_lo", "p", "norms", "send", "slot_offset", "ev", "aux")
+                 "gt_hi", "gt_lo", "f_hi", "f_lo", "p", "norms", "send", "slot_offset", "ev", "aux", "rows")
 
     def __init__(self, spec):
-        for name, value in zip(self.__slots__, spec, strict=True):
+        for name, value in zip(self.__slots__, (*spec, None) if len(spec) == 23 else spec, strict=True):
             setattr(self, name, value)
+
+    def measure(self, k, x, div=1):
+        """Bounds of the rows of ``x`` into the k-th bounds of a half-pair block (``div`` rows to one)."""
+        if self.rows is not None and self.rows[k] is not None:
+            rows = x.abs().nan_to_num().amax(1).view(-1, div).amax(1)
+            self.rows[k][: len(rows)].copy_(torch.maximum(self.rows[k][: len(rows)], rows))
 
     def w(self):
         """The parameter block as an (m, n) view."""
@@ -89,6 +95,7 @@ class FakeBlockExt(FakeExt):
             A = a_hi + (a_lo if a_lo is not None else 0)
             B = b_hi + (b_lo if b_lo is not None else 0)
             acc = (A.double() @ B.double().T).float()
+            self.check_rows(spec, A, B, None, alpha)
             if flags & self.FLAG_SQUARE_ACC:
                 acc = acc * acc
             if flags & self.FLAG_PACKED_C:
@@ -104,8 +111,10 @@ class FakeBlockExt(FakeExt):
 
     # -- the step's pointwise kernels ------------------------------------------------------------
     def grad_prologue(self, blocks, _tiles, _n, grad_ptrs, l2, beta1, beta3, bc1, graft_kind, g_beta2, g_weight, g_bc2,
-                      g_eps, write_split, status, num_grad_peers, grad_scale):
+                      g_eps, write_split, status, num_grad_peers, grad_scale, filtered_plain=False, scratch=None):
         assert num_grad_peers == 0, "the stand-in has no peers"
+        if scratch is not None:
+            scratch.zero_()
         pointers = grad_ptrs.tolist()
         for b in blocks:
             w = b.w()
@@ -117,6 +126,8 @@ class FakeBlockExt(FakeExt):
                 status[0] |= 2
             if l2 != 0.0:
                 g = g + l2 * w
+            b.measure(0, g)
+            b.measure(1, g.T, b.rows[2] if b.rows is not None else 1)
             if b.g_hi is not None:
                 b.g_hi[:, : b.n].copy_(g)
                 if b.g_lo is not None:
@@ -133,6 +144,8 @@ class FakeBlockExt(FakeExt):
                 old = m1.clone()
                 m1.copy_(torch.lerp(old, g, 1.0 - beta1))
                 f = (torch.lerp(old, g, 1.0 - beta3) if beta3 != beta1 else m1) / bc1
+            b.measure(3, f)
+            b.measure(4, f.T)
             if b.f_hi is not None:
                 b.f_hi[:, : b.n].copy_(f)
                 if b.f_lo is not None:
@@ -212,7 +225,10 @@ class FakeBlockExt(FakeExt):
                 continue
             p = b.p.view(b.m, b.n)
             ev = b.ev.view(b.m, b.n)
-            b.f_hi[:, : b.n].copy_(p / (torch.pow(ev / bc2, inv_root) + eps))
+            scaled = p / (torch.pow(ev / bc2, inv_root) + eps)
+            b.measure(5, scaled)
+            b.measure(6, scaled.T)
+            b.f_hi[:, : b.n].copy_(scaled)
             if b.f_lo is not None:
                 b.f_lo.zero_()
 

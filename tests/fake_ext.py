@@ -5,7 +5,8 @@ of ``optimizers_b200/matrix/eigh_dc.py`` make (launch tables, grouped products w
 flags and operand views, the per-matrix passes, the Householder factorisation, the Jacobi leaves)
 with plain torch on whatever device the tensors live on.  Products are formed in fp64 and rounded
 once, operand pairs are (value, 0): the arithmetic is at least as accurate as the kernels', so a
-test that passes here checks the Python around the kernels, not the kernels.
+test that passes here checks the Python around the kernels, not the kernels.  Arrays of half pairs hold the fp32 values
+themselves, in the padded layout of the pairs; every product that is given bounds of their rows checks them.
 """
 
 import torch
@@ -13,7 +14,8 @@ import torch
 
 class FakeExt:
     FLAG_PACKED_C, FLAG_SPLIT_OUT, FLAG_SUMSQ, FLAG_NO_C = 1, 2, 4, 8
-    FLAG_MIRROR, FLAG_ADD_DIAG, FLAG_TRACE = 64, 128, 256
+    FLAG_MIRROR, FLAG_ADD_DIAG, FLAG_TRACE, FLAG_FIXED_SCALE = 64, 128, 256, 512
+    HALF_PAIR, HALF_PAIR_SYM = 2, 3
 
     def __init__(self):
         self.gemm_launches = 0
@@ -34,6 +36,61 @@ class FakeExt:
             out.append(tuple(views))
         return out
 
+    def alloc_pair_batch(self, sizes, device):
+        return [torch.full((n, (n + 31) // 32 * 32), float("nan"), device=device) for n in sizes]
+
+    # -- bounds of chained products ----------------------------------------------------------------
+    def build_row_bound_table(self, specs):
+        return list(specs)
+
+    def row_bounds(self, specs):
+        for mat, rows, vec, out, top in specs:
+            d = mat.shape[0]
+            assert bool((mat.abs().amax(1) <= rows[:d]).all())
+            assert vec.numel() >= mat.shape[1] and not vec[d : mat.shape[1]].any()
+            out[:d].copy_(1.001 * (mat[:, :d].abs() @ vec[:d]))
+            if top is not None:
+                top.copy_(torch.maximum(top, out[:d].max()))
+
+    # -- mirrors as half pairs -------------------------------------------------------------------
+    def build_pair_table(self, specs):
+        return (list(specs), None, 0, None, 0)
+
+    def pair_mirrors(self, specs, *_):
+        for src, dst, bounds, dst_t, *bounds_t in specs:
+            d = src.shape[0]
+            value = src.clone()
+            for out, x, to in ((dst, value, bounds), (dst_t, value.T, bounds_t[0] if bounds_t else None)):
+                if out is None:
+                    continue
+                assert out.shape[1] == (d + 31) // 32 * 32
+                out[:d, :d].copy_(x)
+                out[:d, d:].zero_()
+                rows, l1, top = to
+                rows[:d].copy_(x.abs().amax(1))
+                if l1 is not None:
+                    l1[:d].copy_(x.abs().sum(1))
+                if top is not None:
+                    assert float(top) == 0.0
+                    top.copy_(x.abs().sum(1).max())
+
+    def check_rows(self, spec, A, B, result, alpha):
+        """The bounds a half-pair product is given hold, and those of its result are written and hold."""
+        if len(spec) < 15 or spec[14] is None:
+            return
+        a_bound, a_div, b_bound, b_div, out = spec[14]
+        assert A.shape[1] % 32 == 0 and A.is_contiguous() and B.is_contiguous()
+        for x, bound, div in ((A, a_bound, a_div), (B, b_bound, b_div)):
+            limit = bound[torch.arange(x.shape[0]) // div]
+            assert bool((torch.nan_to_num(x).abs().amax(1) <= limit).all()), "an operand row exceeds its bound"
+        if out is None or spec[6] is not None:
+            return
+        left, right, cap, bound = out
+        if left is not None:
+            bound[: A.shape[0]].copy_(abs(alpha) * (left[: A.shape[0]] * right).clamp(max=float("inf") if cap is None else float(cap)))
+        limit = bound[torch.zeros(A.shape[0], dtype=torch.long) if bound.numel() == 1 else torch.arange(A.shape[0])]
+        assert bool((torch.nan_to_num(result).abs().amax(1) <= limit * (1 + 1e-5)).all()), "a result exceeds its bound"
+
     # -- operand split -------------------------------------------------------------------------
     def tf32_split(self, src, hi, lo):
         hi.copy_(src)
@@ -50,7 +107,7 @@ class FakeExt:
             a_hi, a_lo, b_hi, b_lo, c, d_hi, d_lo, sumsq, _ldc, _ldd, flags, upper = spec[:12]
             A = a_hi + (a_lo if a_lo is not None else 0)
             B = b_hi + (b_lo if b_lo is not None else 0)
-            if len(spec) == 14 and spec[13] is not None:
+            if len(spec) >= 14 and spec[13] is not None:
                 ar, ak, br, bk, M, N, K = spec[13]
                 A, B = A[ar : ar + M, ak : ak + K], B[br : br + N, bk : bk + K]
             assert A.shape[1] == B.shape[1], (A.shape, B.shape)
@@ -63,6 +120,7 @@ class FakeExt:
                 out = out + beta * c[:m, :n]
             if flags & self.FLAG_ADD_DIAG:
                 out = out + gamma * torch.eye(m, n)
+            self.check_rows(spec, a_hi, b_hi, out, alpha)
             if flags & self.FLAG_SUMSQ:
                 sumsq[0] += (out.double() ** 2).sum().float()
             if flags & self.FLAG_TRACE:
@@ -71,7 +129,10 @@ class FakeExt:
                 c[:m, :n].copy_(out)
             if flags & self.FLAG_SPLIT_OUT:
                 d_hi[:m, :n].copy_(out)
-                d_lo[:m, :n].zero_()
+                if d_lo is not None:
+                    d_lo[:m, :n].zero_()
+                else:  # half pairs: whole chunks
+                    d_hi[:m, n : (n + 31) // 32 * 32].zero_()
 
     # -- coupled iterations ----------------------------------------------------------------------
     def build_mat_table(self, specs):

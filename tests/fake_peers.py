@@ -94,22 +94,23 @@ class FakePeerExt(FakeBlockExt):
             ctypes.memmove(destination, source, nbytes)
 
     def grad_prologue(self, blocks, tiles, n, grad_ptrs, l2, beta1, beta3, bc1, graft_kind, g_beta2, g_weight, g_bc2, g_eps,
-                      write_split, status, num_grad_peers, grad_scale):
+                      write_split, status, num_grad_peers, grad_scale, filtered_plain=False, scratch=None):
         if num_grad_peers == 0:
             return super().grad_prologue(blocks, tiles, n, grad_ptrs, l2, beta1, beta3, bc1, graft_kind, g_beta2, g_weight,
-                                         g_bc2, g_eps, write_split, status, 0, grad_scale)
+                                         g_bc2, g_eps, write_split, status, 0, grad_scale, filtered_plain, scratch)
+        assert scratch is None and write_split != self.HALF_PAIR  # a gradient summed from the peers is not on half pairs
         # The owner sums the peers' gradients in rank order and scales the sum: build that gradient
         # in a scratch tensor per slot and hand the local form a table pointing at the scratch.
         pointers = grad_ptrs.tolist()
         slots = sorted({b.grad_slot for b in blocks})
-        scratch, table = {}, [0] * (max(slots) + 1)
+        sums, table = {}, [0] * (max(slots) + 1)
         for slot in slots:
             extent = max((b.grad_offset + (b.m - 1) * b.w().stride(0) + b.n) for b in blocks if b.grad_slot == slot)
             total = torch.zeros(extent)
             for r in range(num_grad_peers):
                 total += _at(pointers[slot * num_grad_peers + r], extent)
-            scratch[slot] = total * grad_scale
-            table[slot] = scratch[slot].data_ptr()
+            sums[slot] = total * grad_scale
+            table[slot] = sums[slot].data_ptr()
         return super().grad_prologue(blocks, tiles, n, torch.tensor(table, dtype=torch.int64), l2, beta1, beta3, bc1, graft_kind,
                                      g_beta2, g_weight, g_bc2, g_eps, write_split, status, 0, 1.0)
 
@@ -144,6 +145,7 @@ class FakePeerExt(FakeBlockExt):
             A = a_hi + (a_lo if a_lo is not None else 0)
             B = b_hi + (b_lo if b_lo is not None else 0)
             out = alpha * (A.double() @ B.double().T).float()
+            self.check_rows(spec, A, B, None, alpha)
             if flags & self.FLAG_SUMSQ:
                 sumsq[0] += (out.double() ** 2).sum().float()
             flat = out.reshape(-1).to(_DTYPES[send_dtype])

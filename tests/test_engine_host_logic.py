@@ -39,10 +39,11 @@ class _Stream(_Event):
         pass
 
 
-def install_cpu_engine(setattr_):
+def install_cpu_engine(setattr_, half_pairs=True):
     """Make ``backend="native"`` build the engine for CPU parameters on top of the stand-in.
     ``setattr_(object, name, value)`` does the patching (pytest's monkeypatch, or plain ``setattr``
-    inside a spawned rank)."""
+    inside a spawned rank).  ``half_pairs=False`` keeps the step's products on tf32 pairs, as in groups that
+    half pairs do not cover."""
     import optimizers_b200.native_engine as engine_module
     from optimizers_b200.ops import build
 
@@ -53,6 +54,8 @@ def install_cpu_engine(setattr_):
         engine_module, "maybe_build_native_engine",
         lambda optimizer, rec, group, cfg: None if cfg.backend == "torch" else engine_module.build_native_engine(optimizer, rec, group, cfg),
     )
+    if not half_pairs:
+        setattr_(engine_module.NativeGroupEngine, "_half_pairs_cover", lambda self, group, cfg: False)
     setattr_(torch.cuda, "Event", _Event)
     setattr_(torch.cuda, "get_device_capability", lambda device=None: (10, 0))
     setattr_(torch.cuda, "current_stream", lambda device=None: _Stream())
@@ -62,7 +65,7 @@ def install_cpu_engine(setattr_):
 
 @pytest.fixture
 def cpu_engine(monkeypatch):
-    return install_cpu_engine(monkeypatch.setattr)
+    return install_cpu_engine(monkeypatch.setattr, half_pairs=False)
 
 
 def _model():
