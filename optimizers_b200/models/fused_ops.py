@@ -103,8 +103,10 @@ class _LMHeadXent(torch.autograd.Function):
 
 def _scaled(product: Tensor, scale: Tensor, dtype: torch.dtype) -> Tensor:
     """``scale`` times a bf16 product in ``dtype`` (fp32 without a rounding to bf16 in between).  A backward
-    that is itself recorded (``create_graph``) keeps to differentiable operations."""
-    if dtype not in (torch.float32, torch.bfloat16) or torch.is_grad_enabled():
+    that is itself recorded (``create_graph``) keeps to differentiable operations, and one that takes a batch of incoming
+    gradients (``is_grads_batched``, ``vmap``) to operations that know of it."""
+    plain = torch._C._has_storage(scale) and torch._C._has_storage(product)  # wrappers of batched tensors have none
+    if dtype not in (torch.float32, torch.bfloat16) or torch.is_grad_enabled() or not plain:
         return (product * scale).to(dtype)
     _count()
     return _ext().scale_cast(product, scale, dtype == torch.bfloat16)

@@ -30,3 +30,22 @@ def test_lm_head_loss_backward_can_be_recorded():
     seed = torch.ones((), device="cuda", requires_grad=True)
     (dw,) = torch.autograd.grad(loss, (w,), grad_outputs=seed, create_graph=True)
     assert dw.requires_grad
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_lm_head_loss_backward_takes_a_batch_of_incoming_gradients(dtype):
+    from optimizers_b200.models.fused_ops import lm_head_cross_entropy
+
+    torch.manual_seed(0)
+    x = torch.randn(32, 64, device="cuda").bfloat16().requires_grad_(True)
+    w = (0.1 * torch.randn(100, 64, device="cuda")).to(dtype).requires_grad_(True)
+    t = torch.randint(0, 100, (32,), device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        loss = lm_head_cross_entropy(x, w, t)
+    seeds = torch.tensor([1.0, -2.0, 0.5], device="cuda")
+    batched = torch.autograd.grad(loss, (x, w), grad_outputs=seeds, is_grads_batched=True, retain_graph=True)
+    single = torch.autograd.grad(loss, (x, w))
+    for many, one in zip(batched, single, strict=True):
+        assert many.dtype == one.dtype and many.shape == (3, *one.shape)
+        for seed, got in zip(seeds, many, strict=True):  # one more rounding to bf16
+            assert float((got.float() - seed * one.float()).norm() / (seed * one.float()).norm()) < 2.0**-8
