@@ -405,7 +405,7 @@ def _more_options(lib):
 
 
 @pytest.mark.skipif(not reference_available(), reason="reference not installed")
-@pytest.mark.parametrize("name", list(_more_options(ob)))
+@pytest.mark.parametrize("name", list(_more_options(ob)) if reference_available() else [])
 def test_more_option_sets_match_reference_bitwise(name):
     """Option sets beyond the family x extras grid: the other weight-decay types, no bias correction,
     plain momentum, no grafting, dims switched off by an exponent of 0 (one side, or the whole
