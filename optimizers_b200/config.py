@@ -718,8 +718,9 @@ class NativeRuntimeConfig:
     backend:   ``"auto"`` uses the native kernels for CUDA parameter groups whose configuration
                they cover and the torch path otherwise; ``"torch"`` forces the torch path;
                ``"native"`` raises if a group cannot run natively.
-    gemm_mode: ``"tf32x3"`` splits fp32 operands into two terms of 11 bits (tf32, or scaled fp16 where the
-               layouts allow it, which has the smaller error) and issues three tensor-core
+    gemm_mode: ``"tf32x3"`` splits fp32 operands into two terms of 11 bits (tf32, or fp16 with a
+               scale per row where the layouts allow it: the smaller error for entries above 2^-28 of their row's
+               largest, 2^-50 of that below) and issues three tensor-core
                products (fp32-grade accuracy); ``"tf32"`` issues one (relative error of a product
                about 1e-3) and keeps one operand array instead of a (hi, lo) pair, which halves the
                engine's operand arrays and mirrors (``DistributedShampoo.native_memory_report()``).

@@ -48,7 +48,8 @@ struct PanelScratch {
   float tau[kQrPanel];
 };
 
-// The panel factorisation of householder_panel_kernel below with the panel in registers: thread t holds rows t,
+// The panel factorisation of householder_panel_kernel below with the panel in registers (but for about 140 bytes a
+// thread that the longest form spills): thread t holds rows t,
 // t + 512, ... (R of them, L <= 512 R) of all 16 columns.  A column step is bound by its chain of
 // latencies (inner products, reduction over the block, pivot, update), so what it touches is kept close: the
 // inner products and the update run on registers, 16 sums take 16 shuffles, every warp adds up the warps'
