@@ -241,3 +241,27 @@ def test_rows_of_a_view_share_the_bound_of_the_row_they_were_written_with(ext):
     assert float(((c.double() - ref).norm(dim=0) / ref.norm(dim=0)).max()) < _bound(64)
     with pytest.raises(RuntimeError, match="a bound per row"):
         ext.build_gemm_plan([(*spec, (a_bound, 1, b_bound, 5, None))])
+
+
+# One tile, ragged tiles, a K loop cut among CTAs, wide tiles; two buffers of this GPU stand in for two ranks'.
+@pytest.mark.parametrize("M,N,K", [(10, 77, 33), (3, 5, 98304), (130, 40, 5000), (2100, 2100, 40)])
+@pytest.mark.parametrize("dtype,code", [(torch.float32, 0), (torch.bfloat16, 1), (torch.float16, 2)])
+def test_pushed_products_on_pairs_are_the_stored_ones(ext, M, N, K, dtype, code):
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    (a, a_bound), (b, b_bound) = (_pairs(torch.randn(n, K, device="cuda", generator=gen) * 0.1) for n in (M, N))
+    status, norm, pushed_norm = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda")
+    c = torch.zeros(M, N, device="cuda")
+    offset = 64  # elements in front of the problem's slot
+    buffers = [torch.full((offset + M * N + 8,), 7.0, device="cuda", dtype=dtype) for _ in range(2)]
+    bounds = (a_bound, 1, b_bound, 1, None)
+    plain = ext.build_gemm_plan([(a, None, b, None, c, None, None, norm, N, 0, ext.FLAG_SUMSQ, False, None, None, bounds)])
+    flags = ext.FLAG_SUMSQ | ext.FLAG_NO_C | ext.FLAG_PEER_PUSH
+    push = ext.build_gemm_plan([(a, None, b, None, None, None, None, pushed_norm, N, 0, flags, False, offset * buffers[0].element_size(), None, bounds)])
+    ext.run_gemm_plan(*plain, 1.0, 0.0, ext.HALF_PAIR, status)
+    for _ in range(2):
+        ext.run_gemm_plan_push(*push, 1.0, 0.0, ext.HALF_PAIR, status, [t.data_ptr() for t in buffers], code)
+    for t in buffers:
+        assert torch.equal(t[offset : offset + M * N].view(M, N), c.to(dtype))
+        assert bool((t[:offset] == 7.0).all()) and bool((t[offset + M * N :] == 7.0).all())
+    assert abs(float(pushed_norm) / (2 * float(norm)) - 1) < 1e-5
+    assert int(status) == 0
